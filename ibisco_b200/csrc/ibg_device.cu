@@ -83,6 +83,16 @@ T* dalloc(size_t n, Owned& owned) {
   owned.add(p, n * sizeof(T));
   return (T*)p;
 }
+// The same once the context's streams may have work: the zeroing runs on the
+// default stream, which a non-blocking stream does not wait for, so it is
+// waited for here, before any kernel or copy of those streams touches the
+// array.
+template <typename T>
+T* dalloc_now(size_t n, Owned& owned) {
+  T* p = dalloc<T>(n, owned);
+  CK(cudaStreamSynchronize(cudaStreamLegacy));
+  return p;
+}
 template <typename T>
 T* dupload(const std::vector<T>& h, Owned& owned) {
   T* p = dalloc<T>(h.size(), owned);
@@ -417,9 +427,9 @@ void alloc_cells(ibg_ctx* c, DevList& L, const float* box) {
   if (ncap <= L.cell_cap) return;
   auto& o = c->owned;
   L.cell_cap = (int)ncap;
-  L.cell_count = dalloc<int>(ncap, o);
-  L.cell_start = dalloc<int>(ncap + 1, o);
-  L.cell_fill = dalloc<int>(ncap, o);
+  L.cell_count = dalloc_now<int>(ncap, o);
+  L.cell_start = dalloc_now<int>(ncap + 1, o);
+  L.cell_fill = dalloc_now<int>(ncap, o);
 }
 
 int grid_for(ibg_ctx* c, long long work, int per_sm = 8) {
@@ -546,8 +556,11 @@ void refresh_args(ibg_ctx* c) {
   const void* src;
   if (c->prec == IBG_PREC_FP32_FIXED) { make_args<float>(c); bytes = sizeof(c->af); src = &c->af; }
   else { make_args<double>(c); bytes = sizeof(c->ad); src = &c->ad; }
-  if (!c->dargs) c->dargs = dalloc<unsigned char>(bytes, c->owned);
-  CK(cudaMemcpy(c->dargs, src, bytes, cudaMemcpyHostToDevice));
+  if (!c->dargs) c->dargs = dalloc_now<unsigned char>(bytes, c->owned);
+  // on the context's stream: a small copy on the default stream may still be
+  // on its way when the call returns, and the context's stream does not wait
+  // for that stream
+  CK(cudaMemcpyAsync(c->dargs, src, bytes, cudaMemcpyHostToDevice, c->st));
 }
 
 const BlockMap kOne{nullptr, nullptr};
@@ -847,8 +860,8 @@ int check_device(ibg_ctx* c) {
 // Error bits read from the device: clear them there and report.
 int check_bits(ibg_ctx* c, unsigned bits) {
   if (bits) {
-    unsigned zero = 0;
-    CK(cudaMemcpy(&c->sc->err, &zero, sizeof(unsigned), cudaMemcpyHostToDevice));
+    CK(cudaMemsetAsync(&c->sc->err, 0, sizeof(unsigned), c->st));
+    CK(cudaStreamSynchronize(c->st));
     return fail(c, status_from_bits(bits), bits_message(bits));
   }
   return IBG_OK;
@@ -898,31 +911,32 @@ int grow_lists(ibg_ctx* c) {
     if (need[w] > L.w_cap) {
       const int cap = need[w] + need[w] / 4 + 2;
       if (L.entries) c->owned.release(L.entries);
-      L.entries = dalloc<int>((size_t)L.nslices * 32 * cap, c->owned);
+      L.entries = dalloc_now<int>((size_t)L.nslices * 32 * cap, c->owned);
       L.w_cap = cap;
       ++c->list_growths;
     }
     if (need_near[w] > L.near_cap) {  // pairs at the cutoff (FP32 path)
       const int cap = need_near[w] + need_near[w] / 4 + 64;
       if (L.near) c->owned.release(L.near);
-      L.near = dalloc<int4>(cap, c->owned);
+      L.near = dalloc_now<int4>(cap, c->owned);
       L.near_cap = cap;
     }
   }
-  const int zero[3] = {0, 0, 0};
-  CK(cudaMemcpy(&c->sc->abort, zero, sizeof(int), cudaMemcpyHostToDevice));
-  CK(cudaMemcpy(&c->sc->skip, zero, sizeof(int), cudaMemcpyHostToDevice));
-  CK(cudaMemcpy(c->sc->need_rows, zero, 2 * sizeof(int), cudaMemcpyHostToDevice));
-  CK(cudaMemcpy(c->sc->need_near, zero, 2 * sizeof(int), cudaMemcpyHostToDevice));
-  CK(cudaMemcpy(c->sc->near_n, zero, 2 * sizeof(unsigned), cudaMemcpyHostToDevice));
+  // all on the context's stream, ahead of the repeated step
+  CK(cudaMemsetAsync(&c->sc->abort, 0, sizeof(int), c->st));
+  CK(cudaMemsetAsync(&c->sc->skip, 0, sizeof(int), c->st));
+  CK(cudaMemsetAsync(c->sc->need_rows, 0, 2 * sizeof(int), c->st));
+  CK(cudaMemsetAsync(c->sc->need_near, 0, 2 * sizeof(int), c->st));
+  CK(cudaMemsetAsync(c->sc->near_n, 0, 2 * sizeof(unsigned), c->st));
   // the bonded branch of the aborted step may have run (it overlaps the list
   // build), and so may its nonbonded kernels (a step aborted for the pairs at
   // the cutoff): their sums are recomputed when the step is repeated
-  CK(cudaMemset(c->fb, 0, accsize(c) * 3 * (size_t)c->nitems));
+  CK(cudaMemsetAsync(c->fb, 0, accsize(c) * 3 * (size_t)c->nitems, c->st));
   for (auto& L : c->L)
-    if (L.present) CK(cudaMemset(L.fsort, 0, accsize(c) * fs_len(L.n)));
-  CK(cudaMemset(c->sc->nbacc, 0, sizeof(c->sc->nbacc)));
+    if (L.present) CK(cudaMemsetAsync(L.fsort, 0, accsize(c) * fs_len(L.n), c->st));
+  CK(cudaMemsetAsync(c->sc->nbacc, 0, sizeof(c->sc->nbacc), c->st));
   refresh_args(c);
+  CK(cudaStreamSynchronize(c->st));  // a batch repeats the step on its own stream
   for (auto& kv : c->graphs) cudaGraphExecDestroy(kv.second);  // they bake the old pointers
   c->graphs.clear();
   return 1;
@@ -953,7 +967,7 @@ int ibg_set_list_rows(ibg_ctx* c, int rows) {
     for (auto& L : c->L) {
       if (!L.present) continue;
       if (L.entries) c->owned.release(L.entries);
-      L.entries = dalloc<int>((size_t)L.nslices * 32 * rows, c->owned);
+      L.entries = dalloc_now<int>((size_t)L.nslices * 32 * rows, c->owned);
       L.w_cap = rows;
     }
     refresh_args(c);
@@ -973,7 +987,7 @@ int ibg_set_vsite_com(ibg_ctx* c, int form) {
     c->vs_com_form = form;
     if (form == IBG_VS_COM_REFERENCE && c->nvirta > 0 && !c->vchain) {
       const size_t nb = c->prec == IBG_PREC_FP32_FIXED ? chain_bytes<float>(c->nvirta) : chain_bytes<double>(c->nvirta);
-      c->vchain = dalloc<unsigned char>(nb, c->owned);
+      c->vchain = dalloc_now<unsigned char>(nb, c->owned);
     }
     refresh_args(c);
     for (auto& kv : c->graphs) cudaGraphExecDestroy(kv.second);
@@ -1137,11 +1151,12 @@ int ibg_autotune(ibg_ctx* c, int reps, ibg_tuning* best, ibg_tuning* cand_out, d
     drop_events();
     // the timing launches summed forces and energies: clear them
     for (auto& L : c->L)
-      if (L.present) CK(cudaMemset(L.fsort, 0, accsize(c) * fs_len(L.n)));
-    CK(cudaMemset(c->sc->nbacc, 0, sizeof(c->sc->nbacc)));
-    CK(cudaMemset(c->sc->work, 0, sizeof(c->sc->work)));
+      if (L.present) CK(cudaMemsetAsync(L.fsort, 0, accsize(c) * fs_len(L.n), c->st));
+    CK(cudaMemsetAsync(c->sc->nbacc, 0, sizeof(c->sc->nbacc), c->st));
+    CK(cudaMemsetAsync(c->sc->work, 0, sizeof(c->sc->work), c->st));
     unsigned bits = 0;
-    CK(cudaMemcpy(&bits, &c->sc->err, sizeof(unsigned), cudaMemcpyDeviceToHost));
+    CK(cudaMemcpyAsync(&bits, &c->sc->err, sizeof(unsigned), cudaMemcpyDeviceToHost, c->st));
+    CK(cudaStreamSynchronize(c->st));
     if (bits) {
       ibg_set_tuning(c, &keep);
       return check_device(c);
@@ -1456,7 +1471,7 @@ __global__ void k_state_out(int natoms, int nitems, const double* S, const doubl
 }
 
 float* xfer_buf(ibg_ctx* c) {
-  if (!c->xfer) c->xfer = dalloc<float>(12 * (size_t)c->nitems, c->owned);
+  if (!c->xfer) c->xfer = dalloc_now<float>(12 * (size_t)c->nitems, c->owned);
   return c->xfer;
 }
 
@@ -1504,7 +1519,7 @@ int ibg_set_state(ibg_ctx* c, const float* sxyz, const float* vxyz, const float*
     h.miu = 1.0;
     h.stop_at = INT_MAX;
     h.lam[0] = h.lam[1] = 1.0;
-    CK(cudaMemcpy(c->sc, &h, sizeof(h), cudaMemcpyHostToDevice));
+    CK(cudaMemcpyAsync(c->sc, &h, sizeof(h), cudaMemcpyHostToDevice, c->st));
     for (auto& L : c->L) {
       if (!L.present) continue;
       alloc_cells(c, L, box);
@@ -1563,7 +1578,7 @@ static int run_steps(ibg_ctx* c, int first, int nsteps, ibg_obs* per_step, bool 
     if (per_step && nsteps > c->ring_cap) {
       if (c->ring) c->owned.release(c->ring);
       c->ring_cap = std::max(nsteps, 64);
-      c->ring = dalloc<ObsD>(c->ring_cap, c->owned);
+      c->ring = dalloc_now<ObsD>(c->ring_cap, c->owned);
       refresh_args(c);
       for (auto& kv : c->graphs) cudaGraphExecDestroy(kv.second);
       c->graphs.clear();
