@@ -26,6 +26,7 @@
 #include <memory>
 #include <set>
 #include <string>
+#include <tuple>
 #include <vector>
 
 #include "../../include/ibisco_gpu.h"
@@ -129,11 +130,16 @@ struct DevList {
   // tables of this list
   int *ltab = nullptr, *toff = nullptr, *tndat = nullptr;
   int4* ptab = nullptr;  // per type pair: first row, NDAT, 1/bin bits, table present
+  // FP32 path, tables on one grid (k_nonbonded_f32's UNI; NBArgs::tuni)
+  uint2* pbase = nullptr;
+  float4* tuni = nullptr;
+  float uinv = 0, r2_none = 0;
+  int urows = 0;
+  bool uni = false;
   void *tbin = nullptr, *tinv = nullptr, *tfp = nullptr, *tx = nullptr;
   float4* tcoef = nullptr;  // FP32 path: per row {F - dF e, P - dP e, dF, dP} (NBArgs::tcoef)
   int ntab = 0, nrows = 0;
-  size_t smem = 0;
-  bool use_smem = false;
+  bool use_smem = false;  // tables staged in shared memory (tuning)
   float rlist = 0, rlistsq = 0, rcutsq = 0;
   float rgroupsq = 0;  // FP32 path: outer group of the stored lists (ListArgs::rgroupsq); 0: reference order
   bool mixed = true;   // the list holds particles of more than one label (k_nonbonded_f32's MIXED)
@@ -259,20 +265,17 @@ const char* bits_message(unsigned b) {
   return "unknown device error";
 }
 
-size_t rsize(const ibg_ctx* c) { return c->prec == IBG_PREC_FP32_FIXED ? sizeof(float) : sizeof(double); }
 size_t accsize(const ibg_ctx* c) { return c->prec == IBG_PREC_FP32_FIXED ? sizeof(unsigned long long) : sizeof(double); }
 size_t possize(const ibg_ctx* c) { return c->prec == IBG_PREC_FP32_FIXED ? sizeof(float4) : sizeof(double4); }
 
 // ----------------------------------------------------------- list setup
-// The list form of a list of n particles.  Automatic choice on the FP32 path:
-// slice lists where the per-particle form would use its thread build (lists
-// filling the GPU at a thread per particle), per-particle lists below, where
-// the warp build serves them.  Measured on the 2,000,000-bead melt, lists
-// rebuilt every 10 steps: 1.656 ms a step with slice lists against 1.669 ms.
+// The list form of a list of n particles.  Automatic choice: per-particle
+// lists.  Measured with slice lists beside them, per step with lists rebuilt
+// every 10 steps: the 2,000,000-bead melt 1.473 against 1.721 ms, a
+// 160,000-bead melt 164 against 170 us, the 40,000-bead melt 69.6 against 69.3.
 int list_form_of(const ibg_ctx* c, int n) {
   if (c->prec != IBG_PREC_FP32_FIXED || n >= (1 << 28)) return IBG_LIST_PER_PARTICLE;
-  if (c->list_form == IBG_LIST_AUTO) return n >= kThreadBuildMin * c->nsm ? IBG_LIST_PER_SLICE : IBG_LIST_PER_PARTICLE;
-  return c->list_form;
+  return c->list_form == IBG_LIST_PER_SLICE ? IBG_LIST_PER_SLICE : IBG_LIST_PER_PARTICLE;
 }
 
 void build_list(ibg_ctx* c, const ibg_desc* d, int which) {
@@ -386,7 +389,8 @@ void build_list(ibg_ctx* c, const ibg_desc* d, int which) {
     // k - toff[t]): with u = r/bin - n, the kernel's alpha = (r - X_k)/bin
     // is u - e_k, e_k = X_k/bin - n, so F = F_k + (F_k+1 - F_k) alpha is
     // (F_k - dF e_k) + dF u, and the same for P; computed in FP64 from the
-    // FP32 rows the kernel would otherwise read
+    // FP32 rows the kernel would otherwise read.  F's are scaled by -2^32, the
+    // fixed-point scale of j's share (exact: a power of two)
     std::vector<float4> co(L.nrows, make_float4(0.f, 0.f, 0.f, 0.f));
     for (int t = 0; t < L.ntab; ++t)
       for (int k = toff[t]; k < toff[t + 1]; ++k) {
@@ -395,7 +399,7 @@ void build_list(ibg_ctx* c, const ibg_desc* d, int which) {
         const double df = last ? 0.0 : (double)f1[2 * (size_t)k + 2] - fk;
         const double dp = last ? 0.0 : (double)f1[2 * (size_t)k + 3] - pk;
         const double e = (double)x1[k] * (double)i1[t] - (double)(k - toff[t]);
-        co[k] = make_float4((float)(fk - df * e), (float)(pk - dp * e), (float)df, (float)dp);
+        co[k] = make_float4(-kFixScale * (float)(fk - df * e), (float)(pk - dp * e), -kFixScale * (float)df, (float)dp);
       }
     L.tcoef = dupload(co, o);
     std::vector<int4> pt((size_t)NT * NT);
@@ -407,17 +411,42 @@ void build_list(ibg_ctx* c, const ibg_desc* d, int which) {
       pt[k] = t >= 0 ? make_int4(toff[t], tnd[t], ib, 1) : make_int4(0, 0, 0, 0);
     }
     L.ptab = dupload(pt, o);
+    // one grid for all: every type pair of the list has a table, with the same
+    // 1/bin and rows past the largest r/bin a pair inside the cutoff can have.
+    // The nonbonded kernel then takes a pair's table number from a register
+    // instead of a 16-byte descriptor, and checks no range
+    const double rmax = std::sqrt((double)L.rcutsq * (1.0 + 1e-6)) * (1.0 + 1e-6);
+    L.uni = L.ntab > 0 && L.ntab <= 255 && NT <= 8;
+    for (int ti : types)
+      for (int tj : types) L.uni = L.uni && ltab[(size_t)ti * NT + tj] >= 0;
+    for (int t = 0; t < L.ntab && L.uni; ++t)
+      L.uni = i1[t] == i1[0] && rmax * (double)i1[t] < (double)(tnd[t] + 1);
+    if (L.uni) {
+      L.uinv = i1[0];
+      const int rows = (int)(rmax * (double)L.uinv) + 1;
+      L.urows = rows + 1;
+      const double rn = ((double)rows + 0.5) / (double)L.uinv;  // in the zero row
+      L.r2_none = (float)(rn * rn);
+      std::vector<float4> tu;
+      for (int t = 0; t < L.ntab; ++t) {
+        for (int k = 0; k < rows; ++k) tu.push_back(co[toff[t] + k]);
+        tu.push_back(make_float4(0.f, 0.f, 0.f, 0.f));
+      }
+      L.tuni = dupload(tu, o);
+      std::vector<uint2> pb(NT, make_uint2(0u, 0u));
+      for (int ti = 0; ti < NT; ++ti)
+        for (int tj = 0; tj < NT; ++tj) {
+          const unsigned v = (unsigned)std::max(ltab[(size_t)ti * NT + tj], 0);
+          (tj < 4 ? pb[ti].x : pb[ti].y) |= v << (8 * (tj & 3));
+        }
+      L.pbase = dupload(pb, o);
+    }
   } else {
     L.tfp = dupload(fp, o); L.tx = dupload(xx, o); L.tbin = dupload(bin, o);
   }
-  const size_t rs = rsize(c);
-  L.smem = c->prec == IBG_PREC_FP32_FIXED
-               ? kNbAccBytes + sizeof(int4) * (size_t)NT * NT + sizeof(float4) * (size_t)L.nrows + 64
-               : 9 * 256 * sizeof(double) + rs * 3 * (size_t)L.nrows + 2 * rs * L.ntab +
-                     sizeof(int) * ((size_t)NT * NT + 2 * L.ntab + 1) + 64;
-  // launch defaults (ibg_set_tuning / ibg_autotune change them): the FP32
-  // kernel reads its tables through L1, the FP64 kernel stages them
-  L.use_smem = c->prec != IBG_PREC_FP32_FIXED && L.smem <= 200 * 1024;
+  // launch default: tables read through L1 (staged, the FP64 kernel's launch on
+  // the 40,000-bead melt takes 82 us instead of 59)
+  L.use_smem = false;
 }
 
 void alloc_cells(ibg_ctx* c, DevList& L, const float* box) {
@@ -508,7 +537,7 @@ void make_args(ibg_ctx* c) {
     n.fsort = (acc_t*)L.fsort;
     n.ltab = L.ltab; n.toff = L.toff; n.tndat = L.tndat; n.tbin = (const R*)L.tbin; n.tinv = (const R*)L.tinv;
     n.tfp = (const R*)L.tfp; n.tx = (const R*)L.tx; n.ptab = L.ptab; n.chunk = c->nb_chunk;
-    n.tcoef = L.tcoef;
+    n.tcoef = L.tcoef; n.pbase = L.pbase; n.tuni = L.tuni; n.uinv = L.uinv; n.r2_none = L.r2_none; n.urows = L.urows;
     n.rows = c->nb_rows;
     n.window = c->nb_window;
     n.ntab = L.ntab; n.nrows = L.nrows; n.rcutsq = (R)L.rcutsq;
@@ -636,53 +665,87 @@ void enq_rebuild(ibg_ctx* c, DevList& L, int always) {
 template <typename R, bool B>
 using NBKernel = void (*)(const NBArgs<R>, const NBArgs<R>* const*, const BlockMap);
 
-// The nonbonded kernel of a list: tables staged in shared memory or read
-// through L1 (smem), on the FP32 path whether the list mixes labels, and the
-// list form (DevList::form).  Per-particle lists are built for eight lanes
-// per particle.
-template <typename R, bool B>
-NBKernel<R, B> nb_kernel(bool smem, bool mixed, int form);
-
-template <bool B>
-NBKernel<float, B> nb_kernel_f(bool smem, bool mixed, int form) {
-  if (form == 1) {
-    if (smem) return mixed ? k_nonbonded_slices<true, true, B> : k_nonbonded_slices<true, false, B>;
-    return mixed ? k_nonbonded_slices<false, true, B> : k_nonbonded_slices<false, false, B>;
+// What selects the nonbonded kernel of a list: tables staged in shared memory
+// or read through L1 (smem), on the FP32 path whether the list mixes labels
+// and whether its tables share one grid, the list form (DevList::form) and the
+// threads of a block.  Per-particle lists are built for eight lanes per
+// particle.
+struct NBKey {
+  int mixed, smem, form, uni, nt;
+  bool operator<(const NBKey& o) const {
+    return std::tie(mixed, smem, form, uni, nt) < std::tie(o.mixed, o.smem, o.form, o.uni, o.nt);
   }
-  if (smem) return mixed ? k_nonbonded_f32<true, true, B> : k_nonbonded_f32<true, false, B>;
-  return mixed ? k_nonbonded_f32<false, true, B> : k_nonbonded_f32<false, false, B>;
-}
-template <>
-NBKernel<float, false> nb_kernel<float, false>(bool smem, bool mixed, int form) {
-  return nb_kernel_f<false>(smem, mixed, form);
-}
-template <>
-NBKernel<float, true> nb_kernel<float, true>(bool smem, bool mixed, int form) {
-  return nb_kernel_f<true>(smem, mixed, form);
-}
-template <>
-NBKernel<double, false> nb_kernel<double, false>(bool smem, bool, int) {
-  return smem ? k_nonbonded<double, true, 8, false> : k_nonbonded<double, false, 8, false>;
-}
-template <>
-NBKernel<double, true> nb_kernel<double, true>(bool smem, bool, int) {
-  return smem ? k_nonbonded<double, true, 8, true> : k_nonbonded<double, false, 8, true>;
+  bool operator==(const NBKey& o) const { return !(*this < o) && !(o < *this); }
+};
+// Blocks of 512 threads for one system over lists with tables on one grid:
+// 32 warps per SM as with 256, but twice as many of them share one range of
+// slices, and with it the positions in L1 (160,000-bead melt 101 us a launch
+// against 105, hybrid melt 82 against 85).  A batch hands blocks to systems,
+// and its kernel holds the argument block in shared memory: 384 threads at 80
+// registers, without the 140 bytes of spills it has at 64 (24 mixed jobs 6.39
+// ms per 20 steps against 6.51).
+NBKey nb_key(const DevList& L, bool batch) {
+  return NBKey{L.mixed, L.use_smem, L.form, L.uni, L.form == 0 && L.uni ? (batch ? 384 : 512) : 256};
 }
 
-// Dynamic shared memory of a nonbonded launch over list L.
-size_t nb_smem(const ibg_ctx* c, const DevList& L) {
-  const size_t base = c->prec == IBG_PREC_FP32_FIXED ? (size_t)kNbAccBytes : 9 * 8 * sizeof(double);
-  return L.use_smem ? L.smem : base;
+template <typename R, bool B>
+NBKernel<R, B> nb_kernel(const NBKey& k);
+
+template <bool SMEM, bool MIXED, bool B>
+NBKernel<float, B> nb_kernel_f(const NBKey& k) {
+  if (k.form == 1) return k_nonbonded_slices<SMEM, MIXED, B>;
+  if (!k.uni) return k_nonbonded_f32<SMEM, MIXED, false, B, 256>;
+  return k_nonbonded_f32<SMEM, MIXED, true, B, B ? 384 : 512>;
+}
+template <bool B>
+NBKernel<float, B> nb_kernel_b(const NBKey& k) {
+  if (k.smem) return k.mixed ? nb_kernel_f<true, true, B>(k) : nb_kernel_f<true, false, B>(k);
+  return k.mixed ? nb_kernel_f<false, true, B>(k) : nb_kernel_f<false, false, B>(k);
+}
+template <>
+NBKernel<float, false> nb_kernel<float, false>(const NBKey& k) { return nb_kernel_b<false>(k); }
+template <>
+NBKernel<float, true> nb_kernel<float, true>(const NBKey& k) { return nb_kernel_b<true>(k); }
+template <>
+NBKernel<double, false> nb_kernel<double, false>(const NBKey& k) {
+  return k.smem ? k_nonbonded<double, true, 8, false> : k_nonbonded<double, false, 8, false>;
+}
+template <>
+NBKernel<double, true> nb_kernel<double, true>(const NBKey& k) {
+  return k.smem ? k_nonbonded<double, true, 8, true> : k_nonbonded<double, false, 8, true>;
+}
+
+// Dynamic shared memory of a nonbonded launch over list L: the sums, and the
+// tables when they are staged (smem_limit: the most a launch may ask for).
+constexpr size_t kSmemLimit = 200 * 1024;
+size_t nb_smem_of(const ibg_ctx* c, const DevList& L, const NBKey& k, bool staged) {
+  if (c->prec != IBG_PREC_FP32_FIXED) {
+    const size_t rs = sizeof(double);
+    return staged ? 9 * 256 * sizeof(double) + rs * 3 * (size_t)L.nrows + 2 * rs * L.ntab +
+                        sizeof(int) * ((size_t)c->ntype * c->ntype + 2 * L.ntab + 1) + 64
+                  : 9 * 8 * sizeof(double);
+  }
+  size_t b = (size_t)nb_acc_bytes(L.mixed, k.nt);
+  if (staged) {
+    b += sizeof(int4) * (size_t)c->ntype * c->ntype + 64;
+    b += sizeof(float4) * (k.form == 0 && k.uni ? (size_t)L.ntab * L.urows : (size_t)L.nrows);
+  }
+  return b;
+}
+size_t nb_smem(const ibg_ctx* c, const DevList& L, bool batch) {
+  return nb_smem_of(c, L, nb_key(L, batch), L.use_smem);
 }
 
 // Blocks per SM the nonbonded kernel of list L reaches (after raising its
 // dynamic shared-memory limit when needed).
 template <typename R, bool B>
 int nb_occupancy(const ibg_ctx* c, const DevList& L, size_t sm) {
-  NBKernel<R, B> k = nb_kernel<R, B>(L.use_smem, L.mixed, L.form);
+  (void)c;
+  const NBKey key = nb_key(L, B);
+  NBKernel<R, B> k = nb_kernel<R, B>(key);
   if (sm > 48 * 1024) CK(cudaFuncSetAttribute((const void*)k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
   int per = 0;
-  CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, (const void*)k, 256, sm));
+  CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, (const void*)k, key.nt, sm));
   per = std::max(1, per);
   // L1 and shared memory share each SM's 256 KB: ask for the smallest
   // shared-memory carveout that holds `per` blocks and leave the rest to L1,
@@ -702,16 +765,18 @@ int nb_occupancy(const ibg_ctx* c, const DevList& L, size_t sm) {
 
 template <typename R>
 void nb_configure(ibg_ctx* c, DevList& L) {
-  int per = nb_occupancy<R, false>(c, L, nb_smem(c, L));
-  nb_occupancy<R, true>(c, L, nb_smem(c, L));
+  const int nw = nb_key(L, false).nt / 32;
+  int per = nb_occupancy<R, false>(c, L, nb_smem(c, L, false));
+  nb_occupancy<R, true>(c, L, nb_smem(c, L, true));
   if (c->nb_blocks_per_sm > 0) per = std::min(per, c->nb_blocks_per_sm);
   const long long units = (long long)L.nslices * 4;
-  L.grid_nb = (int)std::max<long long>(1, std::min<long long>((long long)c->nsm * per, (units + 7) / 8));
+  L.grid_nb = (int)std::max<long long>(1, std::min<long long>((long long)c->nsm * per, (units + nw - 1) / nw));
 }
 
 template <typename R>
 void enq_nonbonded(ibg_ctx* c, DevList& L) {
-  launch_pdl(c, nb_kernel<R, false>(L.use_smem, L.mixed, L.form), L.grid_nb, 256, nb_smem(c, L), args<R>(c).nb[L.which],
+  const NBKey key = nb_key(L, false);
+  launch_pdl(c, nb_kernel<R, false>(key), L.grid_nb, key.nt, nb_smem(c, L, false), args<R>(c).nb[L.which],
              (const NBArgs<R>* const*)nullptr, kOne);
   if (c->prec == IBG_PREC_FP32_FIXED)
     launch_pdl(c, k_nb_near<false>, 1, 256, 0, args<float>(c).nb[L.which], (const NBArgs<float>* const*)nullptr, kOne);
@@ -1020,7 +1085,7 @@ int ibg_set_tuning(ibg_ctx* c, const ibg_tuning* t) {
     c->nb_window = c->prec == IBG_PREC_FP32_FIXED ? t->nb_window : 0;
     for (auto& L : c->L) {
       if (!L.present) continue;
-      L.use_smem = t->nb_tables_smem != 0 && L.smem <= 200 * 1024;
+      L.use_smem = t->nb_tables_smem != 0 && nb_smem_of(c, L, nb_key(L, false), true) <= kSmemLimit;
       if (c->prec == IBG_PREC_FP32_FIXED) nb_configure<float>(c, L);
       else nb_configure<double>(c, L);
     }
@@ -1236,6 +1301,12 @@ int ibg_create(const ibg_desc* d, int precision, ibg_ctx** out) {
     CK(cudaEventCreateWithFlags(&c->fork_ev[0], cudaEventDisableTiming));
     CK(cudaEventCreateWithFlags(&c->fork_ev[1], cudaEventDisableTiming));
     c->prec = precision;
+    // launch defaults (ibg_set_tuning / ibg_autotune change them).  FP32 path:
+    // a block's own range of units, the last 24/256 shared out; with every unit
+    // taken from the global counter (0) the nonbonded launch of the
+    // 2,000,000-bead melt takes 1,234 us instead of 871, of a 160,000-bead one
+    // 99 instead of 90
+    c->nb_chunk = precision == IBG_PREC_FP32_FIXED ? 24 : 0;
     c->natoms = d->natoms; c->nvirta = d->nvirta; c->nitems = d->nitems; c->ntype = d->ntype;
     c->numatoms = d->numatoms; c->numbeads = d->numbeads; c->ncoarse = d->ncoarse;
     c->ensemble = d->ensemble; c->nupdate = d->nupdate; c->halt_drift = d->halt_drift; c->nmts = d->nmts;
@@ -1900,8 +1971,7 @@ struct BMap {
 struct NBGroup {
   int T = 1;
   int form = 0;  // list form (DevList::form)
-  bool smem = false;
-  bool mixed = true;  // nonbonded groups: lists of more than one label
+  NBKey key{};   // nonbonded groups
   size_t sm = 0;
   BMap map;
 };
@@ -2012,29 +2082,26 @@ void batch_layout(ibg_batch* b) {
       grp.map = make_map(b, g);
       b->lb[w].push_back(grp);
     }
-    // nonbonded: one group per (labels mixed, smem, list form); the group's
+    // nonbonded: one group per (labels mixed, smem, list form, one grid); the group's
     // resident blocks are shared among its systems in proportion to their
     // work units
-    std::set<std::array<int, 3>> keys;
-    auto key_of = [](const DevList& L) { return std::array<int, 3>{(int)L.mixed, (int)L.use_smem, L.form}; };
+    std::set<NBKey> keys;
     for (size_t s = 0; s < n; ++s)
-      if (b->sys[s]->L[w].present) keys.insert(key_of(b->sys[s]->L[w]));
-    for (auto key : keys) {
+      if (b->sys[s]->L[w].present) keys.insert(nb_key(b->sys[s]->L[w], true));
+    for (const NBKey& key : keys) {
       NBGroup grp;
-      grp.mixed = key[0] != 0;
-      grp.smem = key[1] != 0;
-      grp.form = key[2];
+      grp.key = key;
       double units = 0;
       for (size_t s = 0; s < n; ++s) {
         const DevList& L = b->sys[s]->L[w];
-        if (!(L.present && key_of(L) == key)) continue;
-        grp.sm = std::max(grp.sm, nb_smem(b->sys[s], L));
+        if (!(L.present && nb_key(L, true) == key)) continue;
+        grp.sm = std::max(grp.sm, nb_smem(b->sys[s], L, true));
         units += (double)L.nslices * ((L.w_cap + 7) / 8);
       }
       int per = 1;
       for (size_t s = 0; s < n; ++s) {
         const DevList& L = b->sys[s]->L[w];
-        if (L.present && key_of(L) == key) {
+        if (L.present && nb_key(L, true) == key) {
           per = nb_occupancy<R, true>(b->sys[s], L, grp.sm);
           break;
         }
@@ -2042,7 +2109,7 @@ void batch_layout(ibg_batch* b) {
       const double resident = (double)b->nsm * per;
       for (size_t s = 0; s < n; ++s) {
         const DevList& L = b->sys[s]->L[w];
-        if (!(L.present && key_of(L) == key)) { g[s] = 0; continue; }
+        if (!(L.present && nb_key(L, true) == key)) { g[s] = 0; continue; }
         const double u = (double)L.nslices * ((L.w_cap + 7) / 8);
         g[s] = std::max(1, std::min(L.grid_nb, (int)std::lround(resident * u / std::max(units, 1.0))));
       }
@@ -2106,7 +2173,7 @@ void batch_enqueue(ibg_batch* b, unsigned v) {
   // each list (one block per system with the list, as the cell scan)
   for (int w : {1, 0}) {
     for (const NBGroup& grp : b->nb[w]) {
-      launch_on(st, true, nb_kernel<R, true>(grp.smem, grp.mixed, grp.form), grp.map.grid, 256, grp.sm, NBArgs<R>{},
+      launch_on(st, true, nb_kernel<R, true>(grp.key), grp.map.grid, grp.key.nt, grp.sm, NBArgs<R>{},
                 (const NBArgs<R>* const*)b->t_nb[w], grp.map.m());
       ++n;
     }

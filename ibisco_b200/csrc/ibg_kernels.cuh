@@ -451,6 +451,7 @@ __global__ void k_regrid(__grid_constant__ const ListArgs L0, const ListArgs* co
   for (int c = bk.b * blockDim.x + threadIdx.x; c < L.cell_cap; c += bk.g * blockDim.x) L.cell_count[c] = 0;
   for (int g = bk.b * blockDim.x + threadIdx.x; g < L.nslices; g += bk.g * blockDim.x) L.slice_w[g] = 0;
   if (threadIdx.x || bk.b) return;
+  sc->rows_max[L.which] = 0;
   int nc[3];
   for (int c = 0; c < 3; ++c) {
     if (sizeof(R) == 4) nc[c] = fint(sc->boxf[c] / L.rlist);
@@ -731,6 +732,7 @@ __global__ void __launch_bounds__(256, 4) k_list_build_warp(__grid_constant__ co
   int* late = s_late[warp];
   const int cap = L.w_cap * T;  // entries a slot may hold
   int* exs = s_exs[warp];
+  int most = 0;  // most rows of any particle this lane closed
   for (;;) {
     __syncthreads();  // the previous cell's staging is no longer read
     if (threadIdx.x == 0) s_cell = (int)atomicAdd(&sc->work[2 + L.which], 1u);
@@ -874,6 +876,7 @@ __global__ void __launch_bounds__(256, 4) k_list_build_warp(__grid_constant__ co
         L.counts[s] = cnt;
         if (cnt >= L.maxnab) atomicOr(&sc->err, EB_LIST_OVERFLOW);
         const int rows = (cnt + T - 1) / T;
+        most = max(most, rows);
         atomicMax(&L.slice_w[g], rows);
         if (rows > L.w_cap) {
           atomicMax(&sc->need_rows[L.which], rows);
@@ -884,6 +887,7 @@ __global__ void __launch_bounds__(256, 4) k_list_build_warp(__grid_constant__ co
       __syncwarp();  // exs is rewritten for the next particle
     }
   }
+  if (most > 0) atomicMax(&sc->rows_max[L.which], most);
 }
 
 // NEW_NEIGHBOUR_WITHLIST.f90:34-123 for large lists: a thread builds one
@@ -939,6 +943,7 @@ __global__ void __launch_bounds__(256) k_list_build_thread(__grid_constant__ con
   const int lane = threadIdx.x & 31;
   const int cap = L.w_cap * T;  // entries a slot may hold
   const int nchunks = (L.n + 31) / 32;
+  int most = 0;  // most rows of any particle of this thread
   for (;;) {
     int ch = 0;
     if (lane == 0) ch = (int)atomicAdd(&sc->work[2 + L.which], 1u);
@@ -1014,6 +1019,7 @@ __global__ void __launch_bounds__(256) k_list_build_thread(__grid_constant__ con
     L.counts[s] = cnt;
     if (cnt >= L.maxnab) atomicOr(&sc->err, EB_LIST_OVERFLOW);
     const int rows = (cnt + T - 1) / T;
+    most = max(most, rows);
     atomicMax(&L.slice_w[g], rows);
     if (rows > L.w_cap) {
       atomicMax(&sc->need_rows[L.which], rows);
@@ -1021,6 +1027,8 @@ __global__ void __launch_bounds__(256) k_list_build_thread(__grid_constant__ con
       sc->skip = 1;
     }
   }
+  most = __reduce_max_sync(0xffffffffu, most);
+  if (lane == 0 && most > 0) atomicMax(&sc->rows_max[L.which], most);
 }
 
 // Slice lists (FP32 path, ListArgs/NBArgs form 1).  Slice g is the four
@@ -1087,6 +1095,7 @@ __global__ void __launch_bounds__(256) k_list_build_slices(__grid_constant__ con
   unsigned char* keys = s_key[warp];
   int* off = s_off[warp];
   const int cap = L.w_cap * 32;  // entries a slice may hold
+  int most = 0;  // most rows of any slice of this warp
   for (;;) {
     int g = 0;
     if (lane == 0) g = (int)atomicAdd(&sc->work[2 + L.which], 1u);
@@ -1266,6 +1275,7 @@ __global__ void __launch_bounds__(256) k_list_build_slices(__grid_constant__ con
     }
     // empty entries up to the end of the last row
     const int rows = (cnt + 31) / 32;
+    most = max(most, rows);
     if (cnt + lane < rows * 32 && cnt + lane < cap) L.entries[base + cnt + lane] = 0;
     if (lane < kUSlots && kUSlots * g + lane < L.n) {
       int np = npair[0];
@@ -1284,6 +1294,7 @@ __global__ void __launch_bounds__(256) k_list_build_slices(__grid_constant__ con
     }
     __syncwarp();  // s_ex, buf and keys are rewritten for the next slice
   }
+  if (lane == 0 && most > 0) atomicMax(&sc->rows_max[L.which], most);
 }
 
 // ------------------------------------------------------------- nonbonded
@@ -1312,6 +1323,14 @@ struct NBArgs {
   const R* tbin;
   const R* tinv; // 1/bin per table (FP32 force kernel)
   const int4* ptab;  // FP32 kernel: per type pair {first row, NDAT, 1/bin bits, 1 if a table}
+  // FP32 kernel, UNI (all tables on one grid, 1/bin = uinv): the table numbers
+  // per type, a byte per type of the neighbour, and the coefficient rows of
+  // every table one after another, urows each, F scaled by -2^32; the last of
+  // them is zero and holds r2_none
+  const uint2* pbase;
+  const float4* tuni;
+  float uinv, r2_none;
+  int urows;
   int chunk;         // FP32 kernel: 256ths of the units taken dynamically after the blocks' own ranges (0: all, per warp)
   int window;        // FP32 kernel, chunk > 0: 0 = each block one contiguous range of units; W > 0 = runs of W
                      // consecutive units dealt to the blocks in turn (block b takes runs b, b + G, b + 2G, ...)
@@ -1327,7 +1346,7 @@ struct NBArgs {
   const double* S;
   int natoms;
   const R* tfp;  // 2 per row
-  // FP32 kernel: per row {A, C, B, D}, F = A + B u and P = C + D u with
+  // FP32 kernel: per row {A, C, B, D}, -2^32 F = A + B u and P = C + D u with
   // u = r/bin - (row within the table); one 16-byte read per pair
   const float4* tcoef;
   const R* tx;
@@ -1346,6 +1365,14 @@ __device__ __forceinline__ bool nb_idle(const NBArgs<R>& A) {
     return !(m >= 1 && m <= 3);
   }
   return false;
+}
+
+// Work units of NBArgs::rows rows that cover the longest slice of a list.  (The
+// storage holds a quarter more rows: units counted from it would be empty for
+// every slice.)
+template <typename R>
+__device__ __forceinline__ int nb_units_per_slice(const NBArgs<R>& A) {
+  return max(1, (min(A.sc->rows_max[A.work], A.w_cap) + A.rows - 1) / A.rows);
 }
 
 // NONBONDED_FORCE.F90:45-104.  Persistent grid; a warp owns one slice of
@@ -1405,7 +1432,7 @@ __global__ void __launch_bounds__(256, 4) k_nonbonded(__grid_constant__ const NB
   // work unit = up to ROWS rows of 32 entries of one slice; units are taken
   // dynamically so that warps finish within one unit of each other
   const int ROWS = A.rows;
-  const int U = (A.w_cap + ROWS - 1) / ROWS;
+  const int U = nb_units_per_slice(A);
   const int nunits = A.nslices * U;
   for (;;) {
     int u = 0;
@@ -1507,10 +1534,12 @@ __global__ void __launch_bounds__(256, 4) k_nonbonded(__grid_constant__ const NB
 // 2^(63-S) and above (and Inf/NaN) raise EB_FIXED and count as 0.
 // fabsf(fij) r below 0.99 kFixMax, tested on the force scaled by 2^32
 constexpr float kFixLimScaled = 0.99f * kFixMax * kFixScale;
-// The FP32 nonbonded kernel's energy and virial sums: 9 per pair of lanes of
-// its 256-thread blocks, at the start of its dynamic shared memory.
-constexpr int kNbPairs = 128;
-constexpr int kNbAccBytes = 9 * kNbPairs * (int)sizeof(long long);
+// The FP32 nonbonded kernels' energy and virial sums, at the start of their
+// dynamic shared memory: 7 per lane of their 256-thread blocks for a list of
+// one label, 9 for a list of several.  A lane adds to its own words, with no
+// shuffle and no half-idle warp (per pair of lanes, they took 16 shuffles and
+// nine half-warp updates for every eight list rows).
+__host__ __device__ constexpr int nb_acc_bytes(bool mixed, int nt) { return (mixed ? 9 : 7) * nt * (int)sizeof(long long); }
 
 template <int S>
 __device__ __forceinline__ long long fixq(float v, unsigned& err) {
@@ -1519,60 +1548,85 @@ __device__ __forceinline__ long long fixq(float v, unsigned& err) {
   return __float2ll_rn(s);
 }
 
-// The work units of an FP32 nonbonded launch handed to the warps of a block
-// (NBArgs::chunk, NBArgs::window); unit(u) is called for each of them.
-template <typename F>
-__device__ __forceinline__ void nb_schedule(const NBArgs<float>& A, const Blk& bk, int nunits, F&& unit) {
-  const int lane = threadIdx.x & 31;
-  if (A.chunk > 0) {
-    // each block a contiguous range of units (neighbouring slices), its warps
-    // taking them through a shared counter, so they gather from one region of
-    // space and share it in L1, with no barrier between them; the last
-    // chunk/256 of the units are taken from the global counter by whichever
-    // warps finish their block's range first
-    __shared__ int s_next;
-    if (threadIdx.x == 0) s_next = 0;
-    __syncthreads();
-    const int tail = (int)((long long)nunits * min(A.chunk, 256) / 256);
-    const int nstat = nunits - tail;
-    if (A.window > 0) {
-      // runs of W consecutive units dealt to the blocks in turn: the blocks
-      // advance together through one window of space, whose positions and
-      // force sums then stay in L2, while a block's warps still share a run
+// The sequence of work units one warp of an FP32 nonbonded launch takes
+// (NBArgs::chunk, NBArgs::window): first units of its block's share, taken
+// through a shared counter -- a contiguous range of units (neighbouring
+// slices), or with a window runs of W consecutive units dealt to the blocks in
+// turn --, so that a block's warps gather from one region of space and share
+// it in L1, with no barrier between them; then the last chunk/256 of all units (all of them with chunk 0),
+// taken from a global counter by whichever warps get there first.  A warp
+// knows its next unit while it still works on one, so that it can load ahead.
+struct NbUnits {
+  const NBArgs<float>& A;
+  const Blk& bk;
+  int* own;  // the block's counter, in shared memory
+  int U;     // units per slice
+  int lo, hi;
+  __device__ __forceinline__ NbUnits(const NBArgs<float>& A_, const Blk& bk_, int U_, int* own_)
+      : A(A_), bk(bk_), own(own_), U(U_) {
+    const int ns = nstat();
+    lo = A.window > 0 ? 0 : (int)((long long)ns * bk.b / bk.g);
+    hi = A.window > 0 ? ns : (int)((long long)ns * (bk.b + 1) / bk.g);
+  }
+  // units handed to the blocks; the rest are shared out
+  __device__ __forceinline__ int nstat() const {
+    const int n = A.nslices * U;
+    return A.chunk > 0 ? n - (int)((long long)n * min(A.chunk, 256) / 256) : 0;
+  }
+  // the next unit, -1 when there is none left (every lane of the warp calls)
+  __device__ __forceinline__ int next() {
+    int u = 0;
+    if (lo < hi) {
+      if ((threadIdx.x & 31) == 0) u = atomicAdd(own, 1);
+      u = __shfl_sync(0xffffffffu, u, 0);
       const int W = A.window;
-      for (;;) {
-        int k = 0;
-        if (lane == 0) k = atomicAdd(&s_next, 1);
-        k = __shfl_sync(0xffffffffu, k, 0);
-        const long long u = ((long long)(k / W) * bk.g + bk.b) * W + k % W;
-        if (u >= nstat) break;
-        unit((int)u);
-      }
-    } else {
-      const int lo = (int)((long long)nstat * bk.b / bk.g), hi = (int)((long long)nstat * (bk.b + 1) / bk.g);
-      for (;;) {
-        int k = 0;
-        if (lane == 0) k = atomicAdd(&s_next, 1);
-        k = __shfl_sync(0xffffffffu, k, 0);
-        if (lo + k >= hi) break;
-        unit(lo + k);
-      }
+      const long long v = W > 0 ? ((long long)(u / W) * bk.g + bk.b) * W + u % W : (long long)lo + u;
+      if (v < hi) return (int)v;
+      lo = hi;  // the block's share is taken
     }
-    for (;;) {
-      int u = 0;
-      if (lane == 0) u = nstat + (int)atomicAdd(&A.sc->work[A.work], 1u);
-      u = __shfl_sync(0xffffffffu, u, 0);
-      if (u >= nunits) break;
-      unit(u);
+    if ((threadIdx.x & 31) == 0) u = nstat() + (int)atomicAdd(&A.sc->work[A.work], 1u);
+    u = __shfl_sync(0xffffffffu, u, 0);
+    return u < A.nslices * U ? u : -1;
+  }
+};
+
+// 1/sqrt(x) of a normal x (squared distances are far above the denormals), as
+// rsqrtf gives it there, without rsqrtf's scaling of denormals.
+__device__ __forceinline__ float rsqrt_norm(float x) {
+  float y;
+  asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+  return y;
+}
+
+// The larger of two, NaN if either is.
+__device__ __forceinline__ float max_nan(float a, float b) {
+  float y;
+  asm("max.NaN.f32 %0, %1, %2;" : "=f"(y) : "f"(a), "f"(b));
+  return y;
+}
+
+// v * scale (a power of two) in 2^-24 fixed point, to nearest; saturates
+// outside the 64-bit range (the caller checks the range).
+__device__ __forceinline__ long long fix24(float v, float scale) { return __float2ll_rn(v * (scale * 0x1p24f)); }
+
+// The block's energy and virial sums, [NE + 6][NT] per lane in lacc, into
+// the list's accumulators: V_NB(1..3) and the six virial terms.  With one
+// energy sum (NE = 1) it belongs to the label of the list's particles.
+template <int NE, int NT>
+__device__ __forceinline__ void nb_block_sums(const NBArgs<float>& A, long long* lacc) {
+  constexpr int K = NE + 6;
+  long long acc[K];
+#pragma unroll
+  for (int k = 0; k < K; ++k) acc[k] = lacc[k * NT + threadIdx.x];
+  __syncthreads();
+  block_sum_i64<K>(acc, lacc);
+  if (threadIdx.x < K && lacc[threadIdx.x] != 0) {
+    int to = (int)threadIdx.x + (3 - NE);
+    if (NE == 1 && threadIdx.x == 0) {
+      const int li = A.posq[0].w >> 16;
+      to = li == 1 ? 0 : (li == 2 ? 1 : 2);
     }
-  } else {
-    for (;;) {
-      int u = 0;
-      if (lane == 0) u = (int)atomicAdd(&A.sc->work[A.work], 1u);
-      u = __shfl_sync(0xffffffffu, u, 0);
-      if (u >= nunits) break;
-      unit(u);
-    }
+    atomicAdd(&A.sc->nbacc[A.work][to], (unsigned long long)lacc[threadIdx.x]);
   }
 }
 
@@ -1592,11 +1646,29 @@ __device__ __forceinline__ void nb_schedule(const NBArgs<float>& A, const Blk& b
 // MIXED: the list holds particles of more than one label, so each pair's
 // energy term depends on j's label; otherwise every pair adds to the term of
 // the list's one label.
-template <bool SMEM, bool MIXED, bool B>
-__global__ void __launch_bounds__(256, 4) k_nonbonded_f32(__grid_constant__ const NBArgs<float> A0,
+// UNI: every type pair of the list has a table, all on one grid that reaches
+// past the cutoff, and there are at most eight types (NBArgs::tuni): a pair's
+// table number comes from a packed register, its row is that table's first
+// row plus r/bin, and there is no descriptor to read and no range to check.
+//
+// What bounds it, on the 160,000-bead melt (ncu, one launch): L1 data-pipe
+// wavefronts (70 %; position gathers ~40 %, table rows ~25 %, reductions ~16
+// %) and issue (60 %).  Two rows are evaluated in step so that two positions
+// and two table rows are in flight per lane; a pair that does not count reads
+// a row of zeros instead of branching; lanes keep their own energy and virial
+// sums; the next unit's header is loaded ahead.  58.2 M -> 47 M warp
+// instructions, launch 105 -> 87 us; with blocks of 512 threads and a unit per
+// slice the 2,000,000-bead melt's launch went from 1,131 to 868 us.  Measured
+// and dropped: tables staged in shared memory (99.2 against 99.5 us: random
+// 16-byte rows conflict on banks as they do on L1 tags), positions fetched a
+// row pair ahead (spills at 64 registers, 24 warps at 80: 100 us), units dealt
+// to warps statically (94 against 88 us: uneven slices).
+template <bool SMEM, bool MIXED, bool UNI, bool B, int NT>
+__global__ void __launch_bounds__(NT, 1024 / NT) k_nonbonded_f32(__grid_constant__ const NBArgs<float> A0,
                                                           const NBArgs<float>* const* tab, const BlockMap bm) {
   constexpr int T = 8;  // lanes per particle (the lists are built for eight)
   constexpr int PS = 32 / T;
+  constexpr int NE = MIXED ? 3 : 1;  // energy sums per lane
   pdl_wait();
   pdl_trigger();
   const Blk bk = blk<B>(bm);
@@ -1606,51 +1678,65 @@ __global__ void __launch_bounds__(256, 4) k_nonbonded_f32(__grid_constant__ cons
   Scalars* sc = A.sc;
   if (nb_idle(A)) return;
   extern __shared__ unsigned char smem_raw[];
-  // [9][kNbPairs] sums of each pair of lanes (the two lanes of a pair serve
-  // the same particle): half the shared memory of per-lane sums, which leaves
-  // more of the SM's 256 KB to L1
-  long long* lacc = (long long*)smem_raw;
+  long long* lacc = (long long*)smem_raw;  // [NE + 6][NT] sums of each lane
   // per type pair {first row, last row index, 1/bin bits, has a table}
   const int4* ptab = A.ptab;
-  const float4* tco = A.tcoef;
-  {
-    unsigned char* p = smem_raw + kNbAccBytes;
-    if (SMEM) {
-      int4* s_ptab = (int4*)p;       p += sizeof(int4) * A.ntype * A.ntype;
-      float4* s_co = (float4*)p;
-      for (int k = threadIdx.x; k < A.nrows; k += blockDim.x) s_co[k] = A.tcoef[k];
-      for (int k = threadIdx.x; k < A.ntype * A.ntype; k += blockDim.x) s_ptab[k] = A.ptab[k];
-      ptab = s_ptab; tco = s_co;
-    }
+  const float4* tco = UNI ? A.tuni : A.tcoef;
+  if (SMEM) {
+    unsigned char* p = smem_raw + nb_acc_bytes(MIXED, NT);
+    int4* s_ptab = (int4*)p;       p += sizeof(int4) * A.ntype * A.ntype;
+    float4* s_co = (float4*)p;
+    const int nr = UNI ? A.ntab * A.urows : A.nrows;
+    for (int k = threadIdx.x; k < nr; k += NT) s_co[k] = tco[k];
+    if (!UNI)
+      for (int k = threadIdx.x; k < A.ntype * A.ntype; k += NT) s_ptab[k] = A.ptab[k];
+    ptab = s_ptab; tco = s_co;
   }
-  if (!(threadIdx.x & 1))
-    for (int k = 0; k < 9; ++k) lacc[k * kNbPairs + (threadIdx.x >> 1)] = 0;
+#pragma unroll
+  for (int k = 0; k < NE + 6; ++k) lacc[k * NT + threadIdx.x] = 0;
+  __shared__ int s_next;
+  if (threadIdx.x == 0) s_next = 0;
   __syncthreads();
   // displacement unit per axis: L / 2^32
   const float ux = (float)(sc->box[0] * 0x1p-32), uy = (float)(sc->box[1] * 0x1p-32), uz = (float)(sc->box[2] * 0x1p-32);
   const float2 uxy = make_float2(ux, uy);
+  const float inv = A.uinv;
+  const int urows = A.urows;
+  const float r2_none = A.r2_none, rcut_lo = A.rcut_lo, rcut_hi = A.rcut_hi;
   const int4* pos = A.posq;
   const int lane = threadIdx.x & 31, grp = lane / T, q = lane % T;
   unsigned err = 0;
+  float fmax = 0.f;  // largest |F| r, scaled by 2^32 (NaN stays)
   // a work unit is `rows` list rows of one slice (a multiple of kEnergyRows)
   const int rows = A.rows;
-  const int U = (A.w_cap + rows - 1) / rows;
-  const int nunits = A.nslices * U;
-  long long* la = lacc + (threadIdx.x >> 1);
-  auto unit = [&](int u) {
-    const int g = u / U;
-    const int r0 = (u - g * U) * rows;
-    const int w = min(A.slice_w[g], A.w_cap);
-    if (r0 >= w) return;
-    const int r1 = min(w, r0 + rows);
+  const int U = nb_units_per_slice(A);
+  long long* la = lacc + threadIdx.x;
+  // a unit, the rows of its slice and the lane's particle's list length: what
+  // the next unit's first entries wait for, loaded while the warp works on this one
+  struct Head {
+    int u, w, cnt;
+  };
+  auto head = [&](int u) {
+    const int g = U == 1 ? u : u / U;
     const int s = g * PS + grp;
-    const bool valid = s < A.n;
-    const int cnt = valid ? A.counts[s] : 0;
-    const int* ent = A.entries + (long long)g * A.w_cap * 32 + lane;
-    const int4 pi = valid ? pos[s] : make_int4(0, 0, 0, 0);
-    const int wi = pi.w;
-    const int ti = wi & 0xffff, li = wi >> 16;
+    return Head{u, min(A.slice_w[g], A.w_cap), s < A.n ? A.counts[s] : 0};
+  };
+  auto unit = [&](const Head& h) {
+    const int g = U == 1 ? h.u : h.u / U;
+    const int r0 = (h.u - g * U) * rows, r1 = min(h.w, r0 + rows);
+    if (r0 >= r1) return;
+    const int s = g * PS + grp;
+    // the lane's entries, T per row, and how many are left from the current
+    // row on (a lane without one reads slot 0, which then does not count)
+    const int* e = A.entries + (size_t)g * ((unsigned)A.w_cap * 32u) + (unsigned)(r0 * 32 + lane);
+    int left = min(h.cnt, r1 * T) - r0 * T - q;
+    const bool mine = left > 0;
+    int t0 = left > 0 ? __ldcs(e) : 0, t1 = left > T ? __ldcs(e + 32) : 0;
+    const int4 pi = s < A.n ? pos[s] : make_int4(0, 0, 0, 0);
+    const int ti = pi.w & 0xffff, li = pi.w >> 16;
     const int4* pti = ptab + ti * A.ntype;  // descriptors of (ti, tj) for every tj
+    // UNI: table numbers of (ti, 0..7), a byte each
+    const uint2 pk = UNI ? A.pbase[ti] : make_uint2(0u, 0u);
     // the energy term of a pair follows from j's label once i's is fixed:
     // V_NB(1) when i is an atom, V_NB(3) when i is a virtual site; when i is
     // a bead, V_NB(2) for a bead j and V_NB(3) for a site j
@@ -1662,44 +1748,66 @@ __global__ void __launch_bounds__(256, 4) k_nonbonded_f32(__grid_constant__ cons
     for (int b0 = r0; b0 < r1; b0 += kEnergyRows) {
       const int b1 = min(r1, b0 + kEnergyRows);
       // em: the term of i's label (and bead-bead); e3: bead i with site j.
-      // The virials are summed scaled by -2^32 (exact: a power of two).
-      float em = 0.f, e3 = 0.f;
-      float2 v03 = make_float2(0.f, 0.f), v15 = v03, v24 = v03;  // virial pairs (0,3), (1,5), (2,4)
-      auto pair = [&](int t, const int4& pj) {
-        // nearest image: the wrapped difference of the box fractions (it and
-        // ANINT could choose differently only at |d| = L/2, beyond the cutoff)
-        // packed FP32 pairs (fmul/ffma .f32x2) round each element as the
-        // scalar instructions do
-        const float2 d01 = __fmul2_rn(make_float2((float)(int)((unsigned)pi.x - (unsigned)pj.x),
-                                                  (float)(int)((unsigned)pi.y - (unsigned)pj.y)),
-                                      uxy);
-        const float d0 = d01.x, d1 = d01.y;
-        const float d2 = (float)(int)((unsigned)pi.z - (unsigned)pj.z) * uz;
-        const float r2 = __fmaf_rn(d2, d2, __fmaf_rn(d1, d1, d0 * d0));
-        if (!(r2 < A.rcut_hi)) return;
-        if (r2 > A.rcut_lo) {  // at the cutoff: k_nb_near decides and computes it
-          const unsigned k = atomicAdd(&sc->near_n[A.work], 1u);
-          if (k < (unsigned)A.near_cap) A.near[k] = make_int4(s, t, A.idx[A.sorted[s]], A.idx[A.sorted[t]]);
-          return;  // beyond the buffer: k_nb_near has the step repeated with a larger one
+      // The virials are summed scaled by -2^32 (exact: a power of two):
+      // {xx, yy}, {zx, zy}, yx, zz
+      float em = 0.f, e3 = 0.f, vyx = 0.f, vzz = 0.f;
+      float2 vd = make_float2(0.f, 0.f), vz = vd;
+      struct Geo {
+        float2 d01;
+        float d2, r2;
+      };
+      // nearest image: the wrapped difference of the box fractions (it and
+      // ANINT could choose differently only at |d| = L/2, beyond the cutoff);
+      // packed FP32 pairs (fmul/ffma .f32x2) round each element as the
+      // scalar instructions do
+      auto geo = [&](const int4& pj) {
+        Geo G;
+        G.d01 = __fmul2_rn(make_float2((float)(int)((unsigned)pi.x - (unsigned)pj.x),
+                                       (float)(int)((unsigned)pi.y - (unsigned)pj.y)),
+                           uxy);
+        G.d2 = (float)(int)((unsigned)pi.z - (unsigned)pj.z) * uz;
+        G.r2 = __fmaf_rn(G.d2, G.d2, __fmaf_rn(G.d01.y, G.d01.y, G.d01.x * G.d01.x));
+        return G;
+      };
+      // a pair at the cutoff: k_nb_near decides and computes it (beyond the
+      // buffer, it has the step repeated with a larger one)
+      auto near = [&](const Geo& G, int t) {
+        if (!(G.r2 > rcut_lo && G.r2 < rcut_hi)) return;
+        const unsigned k = atomicAdd(&sc->near_n[A.work], 1u);
+        if (k < (unsigned)A.near_cap) A.near[k] = make_int4(s, t, A.idx[A.sorted[s]], A.idx[A.sorted[t]]);
+      };
+      // a pair's interpolation coefficients {F base, P base, dF, dP}, F scaled
+      // by -2^32 (exact), its r and its weight u.  One that does not count
+      // reads a row of zeros, so that it adds nothing anywhere
+      auto look = [&](float r2, bool in, int wj, float& r, float& u) -> float4 {
+        if (UNI) {
+          r2 = in ? r2 : r2_none;  // in the zero row that ends every table
+          r = r2 * rsqrt_norm(r2);
+          const float rb = r * inv;  // r / bin
+          const int ni = (int)rb;
+          u = rb - (float)ni;
+          const int t = (int)(__byte_perm(pk.x, pk.y, wj & 0x7) & 0xffu);
+          return tco[t * urows + ni];
         }
-        const int wj = pj.w;
-        const int tj = wj & 0xffff, lj = wj >> 16;
-        const int4 pt = pti[tj];
-        const float r = r2 * rsqrtf(r2);
-        const float rb = r * __int_as_float(pt.z);  // r / bin
+        r2 = in ? r2 : 1.f;
+        r = r2 * rsqrt_norm(r2);
+        const int4 pt = pti[wj & 0xffff];
+        const float rb = r * __int_as_float(pt.z);
         int ni = (int)rb;
         // a missing table (all-zero descriptor) or a distance beyond the table
         // stops the step with an error; the row read stays inside the array
         // (it holds at least two rows), so no branch is needed here
-        err |= pt.w ? 0u : (unsigned)EB_MISSING_TABLE;
-        err |= ni > pt.y ? (unsigned)EB_TABLE_RANGE : 0u;
+        err |= !in || pt.w ? 0u : (unsigned)EB_MISSING_TABLE;
+        err |= in && ni > pt.y ? (unsigned)EB_TABLE_RANGE : 0u;
         ni = min(ni, pt.y);
+        u = rb - (float)ni;
+        return in ? tco[pt.x + ni] : make_float4(0.f, 0.f, 0.f, 0.f);
+      };
+      auto pair = [&](const Geo& G, bool in, int t, int wj, const float4& co, float r, float u) {
         // linear interpolation between rows ni and ni + 1 (NONBONDED_FORCE.F90:66-74)
-        const float u = rb - (float)ni;
-        const float4 co = tco[pt.x + ni];  // {F base, P base, dF, dP}
-        const float2 fv = __ffma2_rn(make_float2(co.z, co.w), make_float2(u, u), make_float2(co.x, co.y));
-        const float fij = fv.x, vij = fv.y;
+        const float fs = __fmaf_rn(co.z, u, co.x), vij = __fmaf_rn(co.w, u, co.y);
         if (MIXED) {
+          const int lj = wj >> 16;
           em += (!i_bead || lj == 2) ? vij : 0.f;
           e3 += (i_bead && lj == 3) ? vij : 0.f;
         } else {
@@ -1710,50 +1818,68 @@ __global__ void __launch_bounds__(256, 4) k_nonbonded_f32(__grid_constant__ cons
         // round-to-nearest is symmetric, so i's share is exactly its negation.
         // |f component| <= |fij| r (to rounding): one test keeps every
         // component in range
-        const float fs = fij * -kFixScale;
-        err |= fabsf(fs) * r < kFixLimScaled ? 0u : (unsigned)EB_FIXED;
-        const float2 sxy = __fmul2_rn(make_float2(fs, fs), d01);
-        const float sx = sxy.x, sy = sxy.y, sz = fs * d2;
+        fmax = max_nan(fmax, fabsf(fs) * r);
+        const float sx = fs * G.d01.x, sy = fs * G.d01.y, sz = fs * G.d2;
         const long long qx = __float2ll_rn(sx), qy = __float2ll_rn(sy), qz = __float2ll_rn(sz);
         fi0 -= qx; fi1 -= qy; fi2 -= qz;
-        unsigned long long* fj = (unsigned long long*)A.fsort + fs_at(t);
-        atomicAdd(fj, (unsigned long long)qx);
-        atomicAdd(fj + 32, (unsigned long long)qy);
-        atomicAdd(fj + 64, (unsigned long long)qz);
-        // (xx, yx) += (sx, sy) d0; (yy, zy) += (sy, sz) d1; (zz, zx) += sz (d2, d0)
-        v03 = __ffma2_rn(sxy, make_float2(d0, d0), v03);
-        v15 = __ffma2_rn(make_float2(sy, sz), make_float2(d1, d1), v15);
-        v24 = __ffma2_rn(make_float2(sz, sz), make_float2(d2, d0), v24);
+        if (in) {
+          unsigned long long* fj = (unsigned long long*)A.fsort + fs_at(t);
+          atomicAdd(fj, (unsigned long long)qx);
+          atomicAdd(fj + 32, (unsigned long long)qy);
+          atomicAdd(fj + 64, (unsigned long long)qz);
+        }
+        vd = __ffma2_rn(make_float2(sx, sy), G.d01, vd);
+        vz = __ffma2_rn(make_float2(sz, sz), G.d01, vz);
+        vyx = __fmaf_rn(sy, G.d01.x, vyx);
+        vzz = __fmaf_rn(sz, G.d2, vzz);
       };
-      // list entries are read once per launch: loaded evict-first (__ldcs),
-      // so that the streamed list does not push the positions and force sums
-      // it points into out of L2
+      // two rows per iteration, in step: both positions are gathered before
+      // either distance, both table rows before either force, and the next
+      // two entries are on their way meanwhile.  Entries are read once per
+      // launch: loaded evict-first (__ldcs), so that the streamed list does
+      // not push the positions and force sums it points into out of L2
       for (int it = b0; it < b1; it += 2) {
-        const bool v0 = it * T + q < cnt;
-        const bool v1 = it + 1 < b1 && (it + 1) * T + q < cnt;
-        const int t0 = v0 ? __ldcs(ent + it * 32) : 0;
-        const int t1 = v1 ? __ldcs(ent + (it + 1) * 32) : 0;
-        const int4 p0 = pos[t0];
-        const int4 p1 = pos[t1];
-        if (v0) pair(t0, p0);
-        if (v1) pair(t1, p1);
+        const int4 p0 = pos[(unsigned)t0];
+        const int4 p1 = pos[(unsigned)t1];
+        const bool v0 = left > 0, v1 = left > T;
+        left -= 2 * T;
+        e += 64;
+        const int n0 = left > 0 ? __ldcs(e) : 0;
+        const int n1 = left > T ? __ldcs(e + 32) : 0;
+        const Geo g0 = geo(p0), g1 = geo(p1);
+        const bool in0 = v0 && g0.r2 <= rcut_lo, in1 = v1 && g1.r2 <= rcut_lo;
+        if ((g0.r2 > rcut_lo && g0.r2 < rcut_hi) || (g1.r2 > rcut_lo && g1.r2 < rcut_hi)) {
+          if (v0) near(g0, t0);
+          if (v1) near(g1, t1);
+        }
+        if (in0 || in1) {
+          float r_0, u_0, r_1, u_1;
+          const float4 c0 = look(g0.r2, in0, p0.w, r_0, u_0);
+          const float4 c1 = look(g1.r2, in1, p1.w, r_1, u_1);
+          pair(g0, in0, t0, p0.w, c0, r_0, u_0);
+          pair(g1, in1, t1, p1.w, c1, r_1, u_1);
+        }
+        t0 = n0;
+        t1 = n1;
       }
-      long long v[8];
-      v[0] = fixq<24>(em, err);
-      v[1] = fixq<24>(e3, err);
-      {
-        const float vir[6] = {v03.x, v15.x, v24.x, v03.y, v24.y, v15.y};
-#pragma unroll
-        for (int k = 0; k < 6; ++k) v[2 + k] = fixq<24>(vir[k] * -0x1p-32f, err);
+      // the group's sums, 2^-24 fixed point; |.| of each stays below 2^39
+      float big;
+      if (MIXED) {
+        la[(li == 1 ? 0 : (i_bead ? 1 : 2)) * NT] += fix24(em, 1.f);
+        la[2 * NT] += fix24(e3, 1.f);
+        big = max_nan(fabsf(em), fabsf(e3));
+      } else {
+        la[0] += fix24(em, 1.f);
+        big = fabsf(em);
       }
+      const float vir[6] = {vd.x, vd.y, vzz, vyx, vz.x, vz.y};
+      float bigv = 0.f;
 #pragma unroll
-      for (int k = 0; k < 8; ++k) v[k] += __shfl_xor_sync(0xffffffffu, v[k], 1);
-      if (!(lane & 1)) {
-        la[(li == 1 ? 0 : (i_bead ? 1 : 2)) * kNbPairs] += v[0];
-        la[2 * kNbPairs] += v[1];
-#pragma unroll
-        for (int k = 0; k < 6; ++k) la[(3 + k) * kNbPairs] += v[2 + k];
+      for (int k = 0; k < 6; ++k) {
+        la[(NE + k) * NT] += fix24(vir[k], -0x1p-32f);
+        bigv = max_nan(bigv, fabsf(vir[k]));
       }
+      if (!(big < 0x1p39f && bigv < 0x1p71f)) err |= (unsigned)EB_FIXED;
     }
 #pragma unroll
     for (int o = T / 2; o > 0; o >>= 1) {
@@ -1761,21 +1887,27 @@ __global__ void __launch_bounds__(256, 4) k_nonbonded_f32(__grid_constant__ cons
       fi1 += __shfl_down_sync(0xffffffffu, fi1, o, T);
       fi2 += __shfl_down_sync(0xffffffffu, fi2, o, T);
     }
-    if (q == 0 && valid && r0 * T < cnt) {
+    if (mine && q == 0) {
       unsigned long long* fo = (unsigned long long*)A.fsort + fs_at(s);
       atomicAdd(fo, (unsigned long long)fi0);
       atomicAdd(fo + 32, (unsigned long long)fi1);
       atomicAdd(fo + 64, (unsigned long long)fi2);
     }
   };
-  nb_schedule(A, bk, nunits, unit);
+  NbUnits seq(A, bk, U, &s_next);
+  int u = seq.next();
+  Head h{-1, 0, 0};
+  if (u >= 0) h = head(u);
+  while (h.u >= 0) {
+    u = seq.next();
+    Head hn{-1, 0, 0};
+    if (u >= 0) hn = head(u);
+    unit(h);
+    h = hn;
+  }
+  if (!(fmax < kFixLimScaled)) err |= (unsigned)EB_FIXED;
   if (err) atomicOr(&sc->err, err);
-  long long acc[9];
-  for (int k = 0; k < 9; ++k) acc[k] = (threadIdx.x & 1) ? 0 : lacc[k * kNbPairs + (threadIdx.x >> 1)];
-  __syncthreads();
-  block_sum_i64<9>(acc, lacc);
-  if (threadIdx.x < 9 && lacc[threadIdx.x] != 0)
-    atomicAdd(&sc->nbacc[A.work][threadIdx.x], (unsigned long long)lacc[threadIdx.x]);
+  nb_block_sums<NE, NT>(A, lacc);
 }
 
 // NONBONDED_FORCE.F90:45-104 over slice lists (k_list_build_slices), FP32
@@ -1794,6 +1926,7 @@ __global__ void __launch_bounds__(256, 4) k_nonbonded_f32(__grid_constant__ cons
 template <bool SMEM, bool MIXED, bool B>
 __global__ void __launch_bounds__(256, 3) k_nonbonded_slices(__grid_constant__ const NBArgs<float> A0,
                                                              const NBArgs<float>* const* tab, const BlockMap bm) {
+  constexpr int NE = MIXED ? 3 : 1;  // energy sums per lane
   pdl_wait();
   pdl_trigger();
   const Blk bk = blk<B>(bm);
@@ -1803,11 +1936,11 @@ __global__ void __launch_bounds__(256, 3) k_nonbonded_slices(__grid_constant__ c
   Scalars* sc = A.sc;
   if (nb_idle(A)) return;
   extern __shared__ unsigned char smem_raw[];
-  long long* lacc = (long long*)smem_raw;  // [9][kNbPairs] sums of each pair of lanes
+  long long* lacc = (long long*)smem_raw;  // [NE + 6][256] sums of each lane
   const int4* ptab = A.ptab;
   const float4* tco = A.tcoef;
   {
-    unsigned char* p = smem_raw + kNbAccBytes;
+    unsigned char* p = smem_raw + nb_acc_bytes(MIXED, 256);
     if (SMEM) {
       int4* s_ptab = (int4*)p;       p += sizeof(int4) * A.ntype * A.ntype;
       float4* s_co = (float4*)p;
@@ -1816,8 +1949,8 @@ __global__ void __launch_bounds__(256, 3) k_nonbonded_slices(__grid_constant__ c
       ptab = s_ptab; tco = s_co;
     }
   }
-  if (!(threadIdx.x & 1))
-    for (int k = 0; k < 9; ++k) lacc[k * kNbPairs + (threadIdx.x >> 1)] = 0;
+#pragma unroll
+  for (int k = 0; k < NE + 6; ++k) lacc[k * 256 + threadIdx.x] = 0;
   __syncthreads();
   const float ux = (float)(sc->box[0] * 0x1p-32), uy = (float)(sc->box[1] * 0x1p-32), uz = (float)(sc->box[2] * 0x1p-32);
   const float2 uxy = make_float2(ux, uy);
@@ -1825,9 +1958,8 @@ __global__ void __launch_bounds__(256, 3) k_nonbonded_slices(__grid_constant__ c
   const int lane = threadIdx.x & 31;
   unsigned err = 0;
   const int rows = A.rows;
-  const int U = (A.w_cap + rows - 1) / rows;
-  const int nunits = A.nslices * U;
-  long long* la = lacc + (threadIdx.x >> 1);
+  const int U = nb_units_per_slice(A);
+  long long* la = lacc + threadIdx.x;
   // each warp's slice: the positions of its four particles, read from shared
   // memory by the pair passes (held in registers they push the kernel past
   // its 80-register bound into spills)
@@ -1889,7 +2021,7 @@ __global__ void __launch_bounds__(256, 3) k_nonbonded_slices(__grid_constant__ c
           const float uu = rb - (float)ni;
           const float4 co = tco[pt.x + ni];  // {F base, P base, dF, dP}
           const float2 fv = __ffma2_rn(make_float2(co.z, co.w), make_float2(uu, uu), make_float2(co.x, co.y));
-          const float fij = fv.x, vij = fv.y;
+          const float fs = fv.x, vij = fv.y;  // F scaled by -2^32
           if (MIXED) {
             // V_NB(1) for an atom i, V_NB(3) for a site i or a bead i with a
             // site j, V_NB(2) for two beads
@@ -1899,7 +2031,6 @@ __global__ void __launch_bounds__(256, 3) k_nonbonded_slices(__grid_constant__ c
           } else {
             e1 += vij;
           }
-          const float fs = fij * -kFixScale;
           err |= fabsf(fs) * r < kFixLimScaled ? 0u : (unsigned)EB_FIXED;
           const float2 sxy = __fmul2_rn(make_float2(fs, fs), d01);
           const float sx = sxy.x, sy = sxy.y, sz = fs * d2;
@@ -1930,27 +2061,15 @@ __global__ void __launch_bounds__(256, 3) k_nonbonded_slices(__grid_constant__ c
         entry(ea, pa);
         if (has1) entry(eb, pb);
       }
-      long long v[9];
-      v[0] = fixq<24>(e1, err);
-      v[1] = MIXED ? fixq<24>(e2, err) : 0;
-      v[2] = MIXED ? fixq<24>(e3, err) : 0;
+      la[0] += fixq<24>(e1, err);
+      if (MIXED) {
+        la[256] += fixq<24>(e2, err);
+        la[2 * 256] += fixq<24>(e3, err);
+      }
       {
         const float vir[6] = {v03.x, v15.x, v24.x, v03.y, v24.y, v15.y};
 #pragma unroll
-        for (int k = 0; k < 6; ++k) v[3 + k] = fixq<24>(vir[k] * -0x1p-32f, err);
-      }
-#pragma unroll
-      for (int k = 0; k < 9; ++k) v[k] += __shfl_xor_sync(0xffffffffu, v[k], 1);
-      if (!(lane & 1)) {
-        if (MIXED) {
-#pragma unroll
-          for (int k = 0; k < 3; ++k) la[k * kNbPairs] += v[k];
-        } else {
-          const int li = pi[0].w >> 16;  // the list's one label
-          la[(li == 1 ? 0 : (li == 2 ? 1 : 2)) * kNbPairs] += v[0];
-        }
-#pragma unroll
-        for (int k = 0; k < 6; ++k) la[(3 + k) * kNbPairs] += v[3 + k];
+        for (int k = 0; k < 6; ++k) la[(NE + k) * 256] += fixq<24>(vir[k] * -0x1p-32f, err);
       }
     }
     // the twelve i-force sums over the warp: at each level a lane keeps one
@@ -1981,14 +2100,13 @@ __global__ void __launch_bounds__(256, 3) k_nonbonded_slices(__grid_constant__ c
     }
     __syncwarp();  // pi is rewritten by the next unit
   };
-  nb_schedule(A, bk, nunits, unit);
-  if (err) atomicOr(&sc->err, err);
-  long long acc[9];
-  for (int k = 0; k < 9; ++k) acc[k] = (threadIdx.x & 1) ? 0 : lacc[k * kNbPairs + (threadIdx.x >> 1)];
+  __shared__ int s_next;
+  if (threadIdx.x == 0) s_next = 0;
   __syncthreads();
-  block_sum_i64<9>(acc, lacc);
-  if (threadIdx.x < 9 && lacc[threadIdx.x] != 0)
-    atomicAdd(&sc->nbacc[A.work][threadIdx.x], (unsigned long long)lacc[threadIdx.x]);
+  NbUnits seq(A, bk, U, &s_next);
+  for (int u = seq.next(); u >= 0; u = seq.next()) unit(u);
+  if (err) atomicOr(&sc->err, err);
+  nb_block_sums<NE, 256>(A, lacc);
 }
 
 // Whether the pair of particles gi, gj (FP32 r^2 = r2) lies inside the cutoff as

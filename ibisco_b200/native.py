@@ -442,8 +442,7 @@ class System:
 
     def set_list_form(self, form: int):
         """Verlet-list form of the FP32 path: LIST_AUTO (-1, the default:
-        slice lists for lists of at least 2*64*32 particles per SM),
-        LIST_PER_PARTICLE (0) or LIST_PER_SLICE (1).  The lists are rebuilt by
+        per-particle lists), LIST_PER_PARTICLE (0) or LIST_PER_SLICE (1).  The lists are rebuilt by
         the next set_state, which must follow."""
         self._check(lib().ibg_set_list_form(self._h, int(form)))
 

@@ -227,13 +227,10 @@ int ibg_set_list_rows(ibg_ctx* c, int rows);
    which of the four it pairs with.  Both hold the reference's half-list
    pairs, so ibg_get_neighbour_list returns the same LIST and NNEBS and every
    force sum is bit for bit the same; the slice form gathers each stored
-   neighbour's position and adds its force once per slice.  On the
-   2,000,000-bead melt that cuts the nonbonded kernel's DRAM traffic from
-   1.06 GB to 0.45 GB a launch and its time by 3 %; its list build is slower,
-   and with lists rebuilt every 10 steps a step takes 1.656 ms against
-   1.669 ms (0.0887 against 0.0941 ms on a 40,000-bead melt).  IBG_LIST_AUTO
-   (the default): slice lists for lists of at least 2*64*32 particles per SM
-   of the device (606,208 on 148 SMs), per-particle lists below.  Changing
+   neighbour's position and adds its force once per slice.  Lists rebuilt
+   every 10 steps, a step with per-particle lists takes 1.47 ms on the
+   2,000,000-bead melt (slice lists 1.72 ms) and 164 us on a 160,000-bead one
+   (170 us).  IBG_LIST_AUTO (the default): per-particle lists.  Changing
    the form discards the stored lists: ibg_set_state must be called again
    before the next step.  ibg_get_list_form returns the form in use (of the
    atom list, or of the bead list when there is no atom list):
@@ -244,19 +241,20 @@ int ibg_set_list_rows(ibg_ctx* c, int rows);
 int ibg_set_list_form(ibg_ctx* c, int form);
 int ibg_get_list_form(const ibg_ctx* c);
 /* Launch tuning of the nonbonded kernel: nb_tables_smem stages the tables in
-   shared memory per block (1) or reads them through L1 (0; the FP32 default,
-   the FP64 path stages them); nb_blocks_per_sm limits the resident blocks per
-   SM (0: all that fit); nb_chunk (FP32 path): each block works through its
-   own contiguous range of work units (neighbouring slices), so its warps
-   gather from one region of space, and the last nb_chunk/256 of the units are
-   taken dynamically by whichever warps finish first (0: every warp takes
-   units alone, dynamically); nb_rows: list rows per work unit, 8 or 16 (0:
-   16); nb_window (FP32 path, nb_chunk > 0): 0 gives each block one contiguous
-   range of units, W > 0 deals runs of W consecutive units to the blocks in
-   turn, so that all blocks work through one region of space at a time.  Forces and trajectories do not depend on the tuning (integer force
-   sums); on the FP32 path nonbonded energies and virials are summed in groups
-   of 8 list rows before their exact fixed-point sum, so they do not depend on
-   it either.  Set it before a batch is made of the context.
+   shared memory per block (1) or reads them through L1 (0, the default);
+   nb_blocks_per_sm limits the resident blocks per SM (0: all that fit);
+   nb_chunk (FP32 path; default 24): each block works through its own
+   contiguous range of work units (neighbouring slices), so its warps gather
+   from one region of space, and the last nb_chunk/256 of the units are taken
+   dynamically by whichever warps finish first (0: every warp takes units
+   alone, dynamically); nb_rows: list rows per work unit, 8 or 16 (0: 16);
+   nb_window (FP32 path, nb_chunk > 0): 0 gives each block one contiguous range
+   of units, W > 0 deals runs of W consecutive units to the blocks in turn, so
+   that all blocks work through one region of space at a time.  Forces and
+   trajectories do not depend on the tuning (integer force sums); on the FP32
+   path nonbonded energies and virials are summed in groups of 8 list rows
+   before their exact fixed-point sum, so they do not depend on it either.  Set
+   it before a batch is made of the context.
    ibg_autotune: times each candidate tuning on the context's current lists
    (reps launches each, CUDA events; with an L2 flush set by ibg_set_l2_flush,
    each launch starts from a flushed L2, as a timed step does), keeps the
