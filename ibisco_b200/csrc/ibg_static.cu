@@ -58,14 +58,8 @@ struct StaticArgs {
   float rcutsq;
   unsigned long long* f;  // scratch: 3 * nitems
   double* part;           // scratch: 9 * gridDim.x
-  unsigned* err;          // scratch word after the partials
+  unsigned* err;          // two scratch words after the partials
 };
-
-__global__ void k_static_zero(unsigned long long* f, long long nwords, unsigned* err) {
-  for (long long k = blockIdx.x * (long long)blockDim.x + threadIdx.x; k < nwords; k += (long long)gridDim.x * blockDim.x)
-    f[k] = 0ull;
-  if (blockIdx.x == 0 && threadIdx.x == 0) *err = 0u;
-}
 
 __device__ __forceinline__ long long fixq(float v, unsigned* err) {
   if (!(fabsf(v) < ibg::kFixMax)) {
@@ -75,65 +69,114 @@ __device__ __forceinline__ long long fixq(float v, unsigned* err) {
   return __float2ll_rn(v * ibg::kFixScale);
 }
 
-// One thread per list entry A; REAL*4 arithmetic in the reference's order.
+// T lanes per list entry A, each taking every T-th neighbour, two at a time so
+// that two neighbours' data are in flight; REAL*4 arithmetic in the reference's
+// order.  The forces are exact integer sums, so they do not depend on T.
+//
+// Bound by the latency of its dependent loads (LIST, then the neighbour's
+// position and type, then its table rows): with one thread per A a list of
+// ~50 neighbours was one chain of ~150 of them, and 3,000 particles kept 12
+// blocks busy.  Whole call, a thread per A against 32 and 8 lanes: 3,001
+// particles 154 us, 70, 79; 30,000 146, 96, 104; 60,000 170, 134, 128; 100,000
+// 198, 154, 157.  So a list of fewer than kWideLists particles takes a warp
+// each, a longer one eight lanes (their neighbours share sectors of LIST).
+constexpr int kWideLists = 45000;
+template <int T>
 __global__ void __launch_bounds__(256) k_static_pairs(StaticArgs a) {
   __shared__ double red[9 * 8];
   double acc[9];
 #pragma unroll
   for (int k = 0; k < 9; ++k) acc[k] = 0.0;
-  for (int A = blockIdx.x * blockDim.x + threadIdx.x; A < a.n; A += gridDim.x * blockDim.x) {
-    const int i = a.index_list[A] - 1;
-    if (i < 0 || i >= a.nitems) { atomicOr(a.err, ibg::EB_BAD_INDEX); continue; }
-    const float rx = a.rxyz[3 * i], ry = a.rxyz[3 * i + 1], rz = a.rxyz[3 * i + 2];
-    const int ti = a.itype[i];
-    const int li = a.type_label[i];
-    const bool ti_ok = ti >= 1 && ti <= a.ntype;
-    long long f0 = 0, f1 = 0, f2 = 0;
-    const int cnt = min(a.nnebs[i], a.maxnab);
-    for (int k = 0; k < cnt; ++k) {
-      const int j = a.list[(long long)A * a.maxnab + k] - 1;
-      if (j < 0 || j >= a.nitems) { atomicOr(a.err, ibg::EB_BAD_INDEX); continue; }
-      float d0 = rx - a.rxyz[3 * j], d1 = ry - a.rxyz[3 * j + 1], d2 = rz - a.rxyz[3 * j + 2];
-      d0 = __fsub_rn(d0, __fmul_rn(roundf(__fmul_rn(d0, a.boxinv[0])), a.box[0]));
-      d1 = __fsub_rn(d1, __fmul_rn(roundf(__fmul_rn(d1, a.boxinv[1])), a.box[1]));
-      d2 = __fsub_rn(d2, __fmul_rn(roundf(__fmul_rn(d2, a.boxinv[2])), a.box[2]));
-      const float r2 = __fadd_rn(__fadd_rn(__fmul_rn(d0, d0), __fmul_rn(d1, d1)), __fmul_rn(d2, d2));
-      if (!(r2 < a.rcutsq)) continue;
-      const int tj = a.itype[j];
-      if (!ti_ok || tj < 1 || tj > a.ntype) { atomicOr(a.err, ibg::EB_MISSING_TABLE); continue; }
-      const int tab = a.inbondt[(ti - 1) + a.ntype * (tj - 1)];
-      if (tab < 1 || tab > a.nnbtype) { atomicOr(a.err, ibg::EB_MISSING_TABLE); continue; }
-      const float r = __fsqrt_rn(r2);
-      const float bin = a.binnb[tab - 1];
-      const int ni = (int)__fdiv_rn(r, bin);
-      if (ni < 0 || ni > a.ndatnb[tab - 1] || ni + 1 >= a.ld_nb) { atomicOr(a.err, ibg::EB_TABLE_RANGE); continue; }
-      const long long row = (long long)a.ld_nb * (tab - 1) + ni;
-      const float alpha = __fdiv_rn(__fsub_rn(r, a.rnbond[row]), bin);
-      const float one_a = __fsub_rn(1.0f, alpha);
-      const float fij = __fadd_rn(__fmul_rn(a.nbond_force[row], one_a), __fmul_rn(a.nbond_force[row + 1], alpha));
-      const float vij = __fadd_rn(__fmul_rn(a.nbond_pot[row], one_a), __fmul_rn(a.nbond_pot[row + 1], alpha));
-      if (li == 1) acc[0] += (double)vij;
-      else if (li == 2) {
-        const int lj = a.type_label[j];
-        if (lj == 2) acc[1] += (double)vij;
-        else if (lj == 3) acc[2] += (double)vij;
-      } else if (li == 3) acc[2] += (double)vij;
-      const float fx = __fmul_rn(fij, d0), fy = __fmul_rn(fij, d1), fz = __fmul_rn(fij, d2);
-      const long long qx = fixq(fx, a.err), qy = fixq(fy, a.err), qz = fixq(fz, a.err);
-      f0 += qx; f1 += qy; f2 += qz;
-      atomicAdd(&a.f[3 * (long long)j + 0], (unsigned long long)(-qx));
-      atomicAdd(&a.f[3 * (long long)j + 1], (unsigned long long)(-qy));
-      atomicAdd(&a.f[3 * (long long)j + 2], (unsigned long long)(-qz));
-      acc[3] += (double)__fmul_rn(fx, d0);
-      acc[4] += (double)__fmul_rn(fy, d1);
-      acc[5] += (double)__fmul_rn(fz, d2);
-      acc[6] += (double)__fmul_rn(fy, d0);
-      acc[7] += (double)__fmul_rn(fz, d0);
-      acc[8] += (double)__fmul_rn(fz, d1);
+  const int q = threadIdx.x % T;
+  const int group = (blockIdx.x * blockDim.x + threadIdx.x) / T, ngroups = gridDim.x * (int)blockDim.x / T;
+  // every group of a warp makes the same number of passes (the shuffles below
+  // take the whole warp)
+  const int passes = (a.n + ngroups - 1) / ngroups;
+  for (int p = 0; p < passes; ++p) {
+    const int A = group + p * ngroups;
+    int i = A < a.n ? a.index_list[A] - 1 : -1;
+    if (A < a.n && (i < 0 || i >= a.nitems)) {
+      if (q == 0) atomicOr(a.err, ibg::EB_BAD_INDEX);
+      i = -1;
     }
-    atomicAdd(&a.f[3 * (long long)i + 0], (unsigned long long)f0);
-    atomicAdd(&a.f[3 * (long long)i + 1], (unsigned long long)f1);
-    atomicAdd(&a.f[3 * (long long)i + 2], (unsigned long long)f2);
+    long long f0 = 0, f1 = 0, f2 = 0;
+    if (i >= 0) {
+      const float rx = a.rxyz[3 * i], ry = a.rxyz[3 * i + 1], rz = a.rxyz[3 * i + 2];
+      const int ti = a.itype[i];
+      const int li = a.type_label[i];
+      const bool ti_ok = ti >= 1 && ti <= a.ntype;
+      const int cnt = min(a.nnebs[i], a.maxnab);
+      const int* list = a.list + (long long)A * a.maxnab;
+      auto neighbour = [&](int k) {  // 0-based, -1 when there is none or it is out of range
+        if (k >= cnt) return -1;
+        const int j = list[k] - 1;
+        if (j >= 0 && j < a.nitems) return j;
+        atomicOr(a.err, ibg::EB_BAD_INDEX);
+        return -1;
+      };
+      auto pair = [&](int j, float xj, float yj, float zj, int tj) {
+        float d0 = rx - xj, d1 = ry - yj, d2 = rz - zj;
+        d0 = __fsub_rn(d0, __fmul_rn(roundf(__fmul_rn(d0, a.boxinv[0])), a.box[0]));
+        d1 = __fsub_rn(d1, __fmul_rn(roundf(__fmul_rn(d1, a.boxinv[1])), a.box[1]));
+        d2 = __fsub_rn(d2, __fmul_rn(roundf(__fmul_rn(d2, a.boxinv[2])), a.box[2]));
+        const float r2 = __fadd_rn(__fadd_rn(__fmul_rn(d0, d0), __fmul_rn(d1, d1)), __fmul_rn(d2, d2));
+        if (!(r2 < a.rcutsq)) return;
+        if (!ti_ok || tj < 1 || tj > a.ntype) { atomicOr(a.err, ibg::EB_MISSING_TABLE); return; }
+        const int tab = a.inbondt[(ti - 1) + a.ntype * (tj - 1)];
+        if (tab < 1 || tab > a.nnbtype) { atomicOr(a.err, ibg::EB_MISSING_TABLE); return; }
+        const float r = __fsqrt_rn(r2);
+        const float bin = a.binnb[tab - 1];
+        const int ni = (int)__fdiv_rn(r, bin);
+        if (ni < 0 || ni > a.ndatnb[tab - 1] || ni + 1 >= a.ld_nb) { atomicOr(a.err, ibg::EB_TABLE_RANGE); return; }
+        const long long row = (long long)a.ld_nb * (tab - 1) + ni;
+        const float alpha = __fdiv_rn(__fsub_rn(r, a.rnbond[row]), bin);
+        const float one_a = __fsub_rn(1.0f, alpha);
+        const float fij = __fadd_rn(__fmul_rn(a.nbond_force[row], one_a), __fmul_rn(a.nbond_force[row + 1], alpha));
+        const float vij = __fadd_rn(__fmul_rn(a.nbond_pot[row], one_a), __fmul_rn(a.nbond_pot[row + 1], alpha));
+        if (li == 1) acc[0] += (double)vij;
+        else if (li == 2) {
+          const int lj = a.type_label[j];
+          if (lj == 2) acc[1] += (double)vij;
+          else if (lj == 3) acc[2] += (double)vij;
+        } else if (li == 3) acc[2] += (double)vij;
+        const float fx = __fmul_rn(fij, d0), fy = __fmul_rn(fij, d1), fz = __fmul_rn(fij, d2);
+        const long long qx = fixq(fx, a.err), qy = fixq(fy, a.err), qz = fixq(fz, a.err);
+        f0 += qx; f1 += qy; f2 += qz;
+        atomicAdd(&a.f[3 * (long long)j + 0], (unsigned long long)(-qx));
+        atomicAdd(&a.f[3 * (long long)j + 1], (unsigned long long)(-qy));
+        atomicAdd(&a.f[3 * (long long)j + 2], (unsigned long long)(-qz));
+        acc[3] += (double)__fmul_rn(fx, d0);
+        acc[4] += (double)__fmul_rn(fy, d1);
+        acc[5] += (double)__fmul_rn(fz, d2);
+        acc[6] += (double)__fmul_rn(fy, d0);
+        acc[7] += (double)__fmul_rn(fz, d0);
+        acc[8] += (double)__fmul_rn(fz, d1);
+      };
+      int j0 = neighbour(q), j1 = neighbour(q + T);
+      for (int k = q; k < cnt; k += 2 * T) {
+        // slot 0 stands in for a missing neighbour: its values are not used
+        const int s0 = max(j0, 0), s1 = max(j1, 0);
+        const float x0 = a.rxyz[3 * s0], y0 = a.rxyz[3 * s0 + 1], z0 = a.rxyz[3 * s0 + 2];
+        const float x1 = a.rxyz[3 * s1], y1 = a.rxyz[3 * s1 + 1], z1 = a.rxyz[3 * s1 + 2];
+        const int t0 = a.itype[s0], t1 = a.itype[s1];
+        const int n0 = neighbour(k + 2 * T), n1 = neighbour(k + 3 * T);
+        if (j0 >= 0) pair(j0, x0, y0, z0, t0);
+        if (j1 >= 0) pair(j1, x1, y1, z1, t1);
+        j0 = n0;
+        j1 = n1;
+      }
+    }
+#pragma unroll
+    for (int o = T / 2; o > 0; o >>= 1) {
+      f0 += __shfl_down_sync(0xffffffffu, f0, o, T);
+      f1 += __shfl_down_sync(0xffffffffu, f1, o, T);
+      f2 += __shfl_down_sync(0xffffffffu, f2, o, T);
+    }
+    if (q == 0 && i >= 0) {
+      atomicAdd(&a.f[3 * (long long)i + 0], (unsigned long long)f0);
+      atomicAdd(&a.f[3 * (long long)i + 1], (unsigned long long)f1);
+      atomicAdd(&a.f[3 * (long long)i + 2], (unsigned long long)f2);
+    }
   }
   double out[9];
   ibg::block_sum<9>(acc, red, out);
@@ -141,17 +184,30 @@ __global__ void __launch_bounds__(256) k_static_pairs(StaticArgs a) {
     for (int k = 0; k < 9; ++k) a.part[9 * blockIdx.x + k] = out[k];
 }
 
-// Forces to FP64 (3,NITEMS) and the block partials, in block order, to
-// V_NB(1..3), PT11, PT22, PT33, PT12, PT13, PT23.
-__global__ void k_static_finish(const unsigned long long* f, const double* part, int nblocks, int nitems,
-                                double* fxyz, double* sums) {
+// Forces to FP64 (3,NITEMS) and the block partials to V_NB(1..3), PT11, PT22,
+// PT33, PT12, PT13, PT23 (each by one warp, its lanes taking every 32nd block
+// in order, then the lanes in a fixed order).  The force sums and the error
+// word are left zero for the next call (the scratch is zero when the library
+// is loaded); the call reads the error from err[1].
+__global__ void __launch_bounds__(256) k_static_finish(unsigned long long* f, const double* part, int nblocks,
+                                                       int nitems, double* fxyz, double* sums, unsigned* err) {
   for (long long k = blockIdx.x * (long long)blockDim.x + threadIdx.x; k < 3LL * nitems;
-       k += (long long)gridDim.x * blockDim.x)
+       k += (long long)gridDim.x * blockDim.x) {
     fxyz[k] = (double)(long long)f[k] * ibg::kFixInv;
-  if (blockIdx.x == 0 && threadIdx.x < 9) {
-    double s = 0.0;
-    for (int b = 0; b < nblocks; ++b) s += part[9 * b + threadIdx.x];
-    sums[threadIdx.x] = s;
+    f[k] = 0ull;
+  }
+  if (blockIdx.x == 0) {
+    const int lane = threadIdx.x & 31;
+    for (int k = threadIdx.x >> 5; k < 9; k += (int)blockDim.x >> 5) {
+      double s = 0.0;
+      for (int b = lane; b < nblocks; b += 32) s += part[9 * b + k];
+      s = ibg::warp_sum(s);
+      if (lane == 0) sums[k] = s;
+    }
+    if (threadIdx.x == 0) {
+      err[1] = err[0];
+      err[0] = 0u;
+    }
   }
 }
 
@@ -209,13 +265,14 @@ extern "C" int ibg_nonbonded_static(int nitems, int n, const float* rxyz, const 
   a.f = (unsigned long long*)base;
   a.part = (double*)((unsigned char*)base + kStaticForceWords * 8);
   a.err = (unsigned*)(a.part + 9LL * kStaticBlocks - 1);  // last partial slot is never a block's
-  const int blocks = (int)std::min<long long>(std::max(1, (n + 255) / 256), kStaticBlocks - 1);
-  k_static_zero<<<std::max(1, std::min(1024, (3 * nitems + 255) / 256)), 256, 0, st>>>(a.f, 3LL * nitems, a.err);
-  k_static_pairs<<<blocks, 256, 0, st>>>(a);
-  k_static_finish<<<std::max(1, std::min(1024, (3 * nitems + 255) / 256)), 256, 0, st>>>(a.f, a.part, blocks,
-                                                                                          nitems, fxyz, sums);
+  const int lanes = n < kWideLists ? 32 : 8;
+  const int blocks = (int)std::min<long long>(std::max(1LL, ((long long)n * lanes + 255) / 256), kStaticBlocks - 1);
+  if (lanes == 32) k_static_pairs<32><<<blocks, 256, 0, st>>>(a);
+  else k_static_pairs<8><<<blocks, 256, 0, st>>>(a);
+  k_static_finish<<<std::max(1, std::min(1024, (3 * nitems + 255) / 256)), 256, 0, st>>>(a.f, a.part, blocks, nitems,
+                                                                                          fxyz, sums, a.err);
   unsigned bits = 0;
-  cudaError_t e = cudaMemcpyAsync(&bits, a.err, sizeof(unsigned), cudaMemcpyDeviceToHost, st);
+  cudaError_t e = cudaMemcpyAsync(&bits, a.err + 1, sizeof(unsigned), cudaMemcpyDeviceToHost, st);
   if (e == cudaSuccess) e = cudaStreamSynchronize(st);
   if (e != cudaSuccess) {
     msg(err, errlen, cudaGetErrorString(e));
