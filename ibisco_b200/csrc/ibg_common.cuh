@@ -127,41 +127,52 @@ __device__ __forceinline__ T warp_sum(T v) {
   return v;
 }
 
-// Deterministic block sum of K values per thread; thread 0 of the block gets
-// the result in out[].  Needs K*32 doubles of shared memory.
-template <int K>
-__device__ __forceinline__ void block_sum(double (&v)[K], double* smem, double* out) {
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = (blockDim.x + 31) >> 5;
+// Sums of K values over a warp's lanes, O the distance of this level's exchange
+// (16 first).  At each level a lane keeps half of its values and adds its
+// partner's share of that half, so that K + 4 exchanges do what 5 K would with
+// one full reduction per value.  Returns which of the K sums the lane holds at
+// the end (in v[0]), -1 for none; every sum ends up on exactly one lane, except
+// that lanes whose levels all ran out of halves hold copies marked -1.
+template <int K, int O, typename T>
+__device__ __forceinline__ int warp_fold(T (&v)[K], int lane, T& out) {
+  if constexpr (O == 0) {
+    static_assert(K == 1, "more values than lanes");
+    out = v[0];
+    return 0;
+  } else if constexpr (K == 1) {
+    T w[1] = {v[0] + __shfl_xor_sync(0xffffffffu, v[0], O)};
+    const int r = warp_fold<1, O / 2, T>(w, lane, out);
+    return (lane & O) ? -1 : r;
+  } else {
+    constexpr int H = (K + 1) / 2;
+    const bool up = (lane & O) != 0;
+    T w[H];
 #pragma unroll
-  for (int k = 0; k < K; ++k) v[k] = warp_sum(v[k]);
-  if (lane == 0)
-    for (int k = 0; k < K; ++k) smem[warp * K + k] = v[k];
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    for (int k = 0; k < K; ++k) {
-      double s = 0.0;
-      for (int w = 0; w < nw; ++w) s += smem[w * K + k];
-      out[k] = s;
+    for (int j = 0; j < H; ++j) {
+      const T lo = v[j], hi = j + H < K ? v[j + H] : (T)0;
+      w[j] = (up ? hi : lo) + __shfl_xor_sync(0xffffffffu, up ? lo : hi, O);
     }
+    int r = warp_fold<H, O / 2, T>(w, lane, out);
+    if (r >= 0 && up) r += H;
+    return r < K ? r : -1;
   }
-  __syncthreads();
 }
 
-// Exact block sum of K 64-bit integers per thread; the results are left in
-// smem[0..K-1] (needs 32 + 32*K entries of shared memory) for every thread.
-template <int K>
-__device__ __forceinline__ void block_sum_i64(long long (&v)[K], long long* smem) {
+// Block sums of K values per thread (K <= 32), left in smem[0..K-1] for every
+// thread; smem holds K entries per warp and K more.  The order of the
+// additions is fixed: the lanes of each warp (warp_fold), then the warps in
+// order, value k by thread k.  (With one reduction per value and one thread
+// adding up the warps, MOVE's 18 sums took ~2 us of its 8 on a small system.)
+template <int K, typename T>
+__device__ __forceinline__ void block_sums(T (&v)[K], T* smem) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = (blockDim.x + 31) >> 5;
-#pragma unroll
-  for (int k = 0; k < K; ++k)
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v[k] += __shfl_down_sync(0xffffffffu, v[k], o);
-  if (lane == 0)
-    for (int k = 0; k < K; ++k) smem[32 + warp * K + k] = v[k];
+  T x;
+  const int k = warp_fold<K, 16, T>(v, lane, x);
+  if (k >= 0) smem[K + warp * K + k] = x;
   __syncthreads();
   if (threadIdx.x < K) {
-    long long s = 0;
-    for (int w = 0; w < nw; ++w) s += smem[32 + w * K + threadIdx.x];
+    T s = 0;
+    for (int w = 0; w < nw; ++w) s += smem[K + w * K + threadIdx.x];
     smem[threadIdx.x] = s;
   }
   __syncthreads();

@@ -498,6 +498,15 @@ SysArgs<float>& args<float>(ibg_ctx* c) { return c->af; }
 template <>
 SysArgs<double>& args<double>(ibg_ctx* c) { return c->ad; }
 
+// Whether k_nb_collect takes a list's pairs at the cutoff along: lists of one
+// slot per thread of its grid (up to 8 blocks of 256 per SM, 303,104 particles),
+// where a block's slots are the ones of its number.  It saves k_nb_near's
+// launch, one block that waits for a few dependent loads (5-8 us a step); the
+// longer lists have hundreds of such pairs, which every block would read.
+bool near_in_collect(const ibg_ctx* c, const DevList& L) {
+  return c->prec == IBG_PREC_FP32_FIXED && L.present && (L.n + 255) / 256 <= c->nsm * 8;
+}
+
 // Fill the argument blocks from the context's current arrays and sizes.
 template <typename R>
 void make_args(ibg_ctx* c) {
@@ -543,10 +552,13 @@ void make_args(ibg_ctx* c) {
     n.ntab = L.ntab; n.nrows = L.nrows; n.rcutsq = (R)L.rcutsq;
     n.rcut_lo = L.rcutsq * (1.0f - 1e-6f);
     n.rcut_hi = L.rcutsq * (1.0f + 1e-6f);
-    n.near = L.near; n.near_cap = L.near_cap;
+    n.near = L.near; n.near_cap = L.near_cap; n.near_in_collect = near_in_collect(c, L);
     n.sorted = L.sorted; n.idx = L.idx; n.S = c->S; n.natoms = c->natoms;
     CollectArgs<R>& k = A.col[w];
     k.sc = sc; k.n = L.n; k.mts = (w == 1 && c->nmts > 0); k.sorted = L.sorted; k.idx = L.idx;
+    k.work = w;
+    k.nb = near_in_collect(c, L) ? (const NBArgs<float>*)((char*)c->dargs + offsetof(SysArgs<float>, nb) + w * sizeof(NBArgs<float>))
+                                 : nullptr;
     k.fsort = (acc_t*)L.fsort; k.fnb = (acc_t*)c->fnb; k.mtsf = (acc_t*)L.mtsf;
   }
   DistArgs<R>& d = A.dist;
@@ -583,9 +595,11 @@ void make_args(ibg_ctx* c) {
 void refresh_args(ibg_ctx* c) {
   size_t bytes;
   const void* src;
-  if (c->prec == IBG_PREC_FP32_FIXED) { make_args<float>(c); bytes = sizeof(c->af); src = &c->af; }
-  else { make_args<double>(c); bytes = sizeof(c->ad); src = &c->ad; }
-  if (!c->dargs) c->dargs = dalloc_now<unsigned char>(bytes, c->owned);
+  const bool f32 = c->prec == IBG_PREC_FP32_FIXED;
+  bytes = f32 ? sizeof(c->af) : sizeof(c->ad);
+  if (!c->dargs) c->dargs = dalloc_now<unsigned char>(bytes, c->owned);  // the arguments point into it
+  if (f32) { make_args<float>(c); src = &c->af; }
+  else { make_args<double>(c); src = &c->ad; }
   // on the context's stream: a small copy on the default stream may still be
   // on its way when the call returns, and the context's stream does not wait
   // for that stream
@@ -723,7 +737,7 @@ size_t nb_smem_of(const ibg_ctx* c, const DevList& L, const NBKey& k, bool stage
     const size_t rs = sizeof(double);
     return staged ? 9 * 256 * sizeof(double) + rs * 3 * (size_t)L.nrows + 2 * rs * L.ntab +
                         sizeof(int) * ((size_t)c->ntype * c->ntype + 2 * L.ntab + 1) + 64
-                  : 9 * 8 * sizeof(double);
+                  : 9 * 9 * sizeof(double);
   }
   size_t b = (size_t)nb_acc_bytes(L.mixed, k.nt);
   if (staged) {
@@ -778,7 +792,7 @@ void enq_nonbonded(ibg_ctx* c, DevList& L) {
   const NBKey key = nb_key(L, false);
   launch_pdl(c, nb_kernel<R, false>(key), L.grid_nb, key.nt, nb_smem(c, L, false), args<R>(c).nb[L.which],
              (const NBArgs<R>* const*)nullptr, kOne);
-  if (c->prec == IBG_PREC_FP32_FIXED)
+  if (c->prec == IBG_PREC_FP32_FIXED && !near_in_collect(c, L))
     launch_pdl(c, k_nb_near<false>, 1, 256, 0, args<float>(c).nb[L.which], (const NBArgs<float>* const*)nullptr, kOne);
 }
 
@@ -805,8 +819,10 @@ template <typename R>
 void enq_move(ibg_ctx* c, int update) {
   MoveArgs<R> M = args<R>(c).move;
   M.update = update;
-  // an ordinary launch: it follows the join with the bonded branch
-  k_move<R, false><<<c->g_mv, 256, 0, c->st>>>(M, nullptr, kOne);
+  // an ordinary launch where it follows the join with the bonded branch
+  const bool joined = c->nb + c->na + c->nt + c->no > 0;
+  launch_on(c->st, c->pdl && !c->timing && !joined, k_move<R, false>, c->g_mv, 256, 0, M,
+            (const MoveArgs<R>* const*)nullptr, kOne);
   ++c->launches;
 }
 
@@ -827,6 +843,10 @@ void enqueue_step(ibg_ctx* c, unsigned v) {
   const int always = 0;  // rebuild kernels follow the step's own flag
   mark(c, 4);
   enq_positions<R>(c, 1);
+  // a system without bonded terms has no bonded branch (its partial sums stay
+  // the zeros they were allocated with), and MOVE then follows the nonbonded
+  // chain directly
+  const bool bonded = c->nb + c->na + c->nt + c->no > 0;
   auto bonded_branch = [&]() {
     mark(c, 2);
     enq_bonded<R>(c);
@@ -834,7 +854,7 @@ void enqueue_step(ibg_ctx* c, unsigned v) {
     enq_distribute<R>(c, 1);
   };
   cudaStream_t main_st = c->st;
-  if (fork) {
+  if (fork && bonded) {
     CK(cudaEventRecord(c->fork_ev[0], main_st));
     CK(cudaStreamWaitEvent(c->st2, c->fork_ev[0], 0));
     c->st = c->st2;
@@ -860,8 +880,10 @@ void enqueue_step(ibg_ctx* c, unsigned v) {
   if (c->L[1].present) enq_collect<R>(c, c->L[1]);
   if (c->L[0].present) enq_collect<R>(c, c->L[0]);
   enq_distribute<R>(c, 0);
-  if (fork) CK(cudaStreamWaitEvent(main_st, c->fork_ev[1], 0));
-  else bonded_branch();
+  if (bonded) {
+    if (fork) CK(cudaStreamWaitEvent(main_st, c->fork_ev[1], 0));
+    else bonded_branch();
+  }
   mark(c, 3);
   if (v & V_FORCE_ONLY) {
     enq_move<R>(c, 0);
@@ -1219,6 +1241,7 @@ int ibg_autotune(ibg_ctx* c, int reps, ibg_tuning* best, ibg_tuning* cand_out, d
       if (L.present) CK(cudaMemsetAsync(L.fsort, 0, accsize(c) * fs_len(L.n), c->st));
     CK(cudaMemsetAsync(c->sc->nbacc, 0, sizeof(c->sc->nbacc), c->st));
     CK(cudaMemsetAsync(c->sc->work, 0, sizeof(c->sc->work), c->st));
+    CK(cudaMemsetAsync(c->sc->near_n, 0, sizeof(c->sc->near_n), c->st));
     unsigned bits = 0;
     CK(cudaMemcpyAsync(&bits, &c->sc->err, sizeof(unsigned), cudaMemcpyDeviceToHost, c->st));
     CK(cudaStreamSynchronize(c->st));
@@ -1996,6 +2019,7 @@ struct ibg_batch {
   std::vector<NBGroup> lb[2];  // list build, by T (smem unused)
   std::vector<NBGroup> nb[2];  // nonbonded, by (T, smem)
   bool any_vs = false, any_list[2] = {false, false};
+  bool any_near[2] = {false, false};  // a list whose pairs at the cutoff take a launch of their own
   bool any_com_carry = false;  // a system with the reference's centre-of-mass chain
   std::map<unsigned, cudaGraphExec_t> graphs;
   long long launches = 0, launches_per_variant[8] = {0};
@@ -2061,6 +2085,8 @@ void batch_layout(ibg_batch* b) {
   b->m_fin = make_map(b, g);
   for (int w = 0; w < 2; ++w) {
     for (size_t s = 0; s < n; ++s) b->any_list[w] |= b->sys[s]->L[w].present;
+    for (size_t s = 0; s < n; ++s)
+      b->any_near[w] |= b->prec == IBG_PREC_FP32_FIXED && b->sys[s]->L[w].present && !near_in_collect(b->sys[s], b->sys[s]->L[w]);
     for (size_t s = 0; s < n; ++s) g[s] = b->sys[s]->L[w].present ? b->sys[s]->g_regrid[w] : 0;
     b->m_regrid[w] = make_map(b, g);
     for (size_t s = 0; s < n; ++s) g[s] = b->sys[s]->L[w].present ? b->sys[s]->g_list[w] : 0;
@@ -2177,7 +2203,7 @@ void batch_enqueue(ibg_batch* b, unsigned v) {
                 (const NBArgs<R>* const*)b->t_nb[w], grp.map.m());
       ++n;
     }
-    if (b->prec == IBG_PREC_FP32_FIXED && b->any_list[w]) {
+    if (b->any_near[w]) {
       launch_on(st, true, k_nb_near<true>, b->m_scan[w].grid, 256, 0, NBArgs<float>{},
                 (const NBArgs<float>* const*)b->t_nb[w], b->m_scan[w].m());
       ++n;

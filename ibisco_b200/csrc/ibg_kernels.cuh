@@ -1341,6 +1341,7 @@ struct NBArgs {
   float rcut_lo, rcut_hi;
   int4* near;          // (i slot, j slot, i global id, j global id) of those pairs
   int near_cap;
+  int near_in_collect;  // k_nb_collect takes those pairs along
   const int* sorted;
   const int* idx;
   const double* S;
@@ -1403,9 +1404,9 @@ __global__ void __launch_bounds__(256, 4) k_nonbonded(__grid_constant__ const NB
   const R* tbin = A.tbin;
   const R* tfp = A.tfp;
   const R* tx = A.tx;
-  double* red = (double*)smem_raw;  // 9 * 8 doubles, reused at the end
+  double* red = (double*)smem_raw;  // 9 * 9 doubles
   if (SMEM) {
-    unsigned char* p = smem_raw + 9 * 8 * sizeof(double);
+    unsigned char* p = smem_raw + 9 * 9 * sizeof(double);
     R* s_fp = (R*)p;               p += sizeof(R) * 2 * A.nrows;
     R* s_x = (R*)p;                p += sizeof(R) * A.nrows;
     R* s_bin = (R*)p;              p += sizeof(R) * A.ntab;
@@ -1523,10 +1524,8 @@ __global__ void __launch_bounds__(256, 4) k_nonbonded(__grid_constant__ const NB
   }
   if (err) atomicOr(&sc->err, err);
   __syncthreads();
-  double out[9];
-  block_sum<9>(acc, red, out);
-  if (threadIdx.x == 0)
-    for (int k = 0; k < 9; ++k) atomicAdd((double*)&sc->nbacc[A.work][k], out[k]);
+  block_sums<9>(acc, red);
+  if (threadIdx.x < 9) atomicAdd((double*)&sc->nbacc[A.work][threadIdx.x], red[threadIdx.x]);
 }
 
 // round(v * 2^S) to the nearest 64-bit integer: the scaling by a power of two
@@ -1619,7 +1618,7 @@ __device__ __forceinline__ void nb_block_sums(const NBArgs<float>& A, long long*
 #pragma unroll
   for (int k = 0; k < K; ++k) acc[k] = lacc[k * NT + threadIdx.x];
   __syncthreads();
-  block_sum_i64<K>(acc, lacc);
+  block_sums<K>(acc, lacc);
   if (threadIdx.x < K && lacc[threadIdx.x] != 0) {
     int to = (int)threadIdx.x + (3 - NE);
     if (NE == 1 && threadIdx.x == 0) {
@@ -2141,12 +2140,63 @@ __device__ bool inside_as_fp64(const NBArgs<float>& A, const Scalars* sc, int gi
   return q < (double)A.rcutsq;
 }
 
-// The pairs the FP32 kernel left at the cutoff: each is decided as the FP64
-// path decides it (inside_as_fp64) and, when inside, computed with the FP32
-// kernel's pair arithmetic; its energy and virial terms go to the system's
-// fixed-point sums one pair at a time.  One block per system and list; the
-// block clears the list's pair count for the next launch.  When more pairs came
-// than the buffer holds, the step is aborted and repeated with a larger one.
+// A pair the FP32 kernel left at the cutoff: decided as the FP64 path decides
+// it (inside_as_fp64) and, when inside, computed with the FP32 kernel's pair
+// arithmetic.  f: i's share of the force in fixed point, e: V_NB(1..3) and the
+// six virial terms.  False when the pair does not count.
+__device__ __noinline__ bool near_pair(const NBArgs<float>& A, const int4& nk, float ux, float uy, float uz, long long (&f)[3],
+                          long long (&e)[9], unsigned& err) {
+  const int4 pi = A.posq[nk.x], pj = A.posq[nk.y];
+  const float d0 = (float)(int)((unsigned)pi.x - (unsigned)pj.x) * ux;
+  const float d1 = (float)(int)((unsigned)pi.y - (unsigned)pj.y) * uy;
+  const float d2 = (float)(int)((unsigned)pi.z - (unsigned)pj.z) * uz;
+  const float r2 = __fmaf_rn(d2, d2, __fmaf_rn(d1, d1, d0 * d0));
+  if (!inside_as_fp64(A, A.sc, nk.z, nk.w, r2)) return false;
+  const int ti = pi.w & 0xffff, li = pi.w >> 16, tj = pj.w & 0xffff, lj = pj.w >> 16;
+  const int4 pt = A.ptab[ti * A.ntype + tj];
+  if (!pt.w) { err |= EB_MISSING_TABLE; return false; }
+  const float r = r2 * rsqrtf(r2);
+  const float ib = __int_as_float(pt.z);
+  const int ni = (int)(r * ib);
+  if (ni > pt.y) { err |= EB_TABLE_RANGE; return false; }
+  const int row = pt.x + ni;
+  const float alpha = (r - A.tx[row]) * ib;
+  const float2 a0 = ((const float2*)A.tfp)[row], a1 = ((const float2*)A.tfp)[row + 1];
+  const float fij = __fmaf_rn(a1.x - a0.x, alpha, a0.x);
+  const float vij = __fmaf_rn(a1.y - a0.y, alpha, a0.y);
+  if (!(fabsf(fij) * r < 0.99f * kFixMax)) { err |= EB_FIXED; return false; }
+  const float fx = fij * d0, fy = fij * d1, fz = fij * d2;
+  f[0] = __float2ll_rn(fx * kFixScale);
+  f[1] = __float2ll_rn(fy * kFixScale);
+  f[2] = __float2ll_rn(fz * kFixScale);
+  const bool lab3 = li == 3 || lj == 3;
+  const long long qe = fixq<24>(vij, err);
+  e[0] = li == 1 ? qe : 0;
+  e[1] = li == 2 && lj == 2 ? qe : 0;
+  e[2] = li != 1 && lab3 ? qe : 0;
+  e[3] = fixq<24>(fx * d0, err);
+  e[4] = fixq<24>(fy * d1, err);
+  e[5] = fixq<24>(fz * d2, err);
+  e[6] = fixq<24>(fy * d0, err);
+  e[7] = fixq<24>(fz * d0, err);
+  e[8] = fixq<24>(fz * d1, err);
+  return true;
+}
+
+// More pairs came at the cutoff than their buffer holds: record the need and
+// abort the step, which the host repeats with a larger buffer (as for the
+// Verlet-list storage).
+__device__ __forceinline__ void near_overflow(Scalars* sc, int work, unsigned n) {
+  sc->need_near[work] = (int)n;
+  sc->near_n[work] = 0u;
+  sc->abort = 1;
+  sc->skip = 1;
+}
+
+// The pairs at the cutoff of a list too long for k_nb_collect to take them
+// along (CollectArgs::nb): their forces to the slot-ordered sums, their energy
+// and virial terms to the system's fixed-point sums.  One block per system and
+// list; the block clears the list's pair count for the next launch.
 template <bool B>
 __global__ void __launch_bounds__(256) k_nb_near(__grid_constant__ const NBArgs<float> A0,
                                                  const NBArgs<float>* const* tab, const BlockMap bm) {
@@ -2155,19 +2205,12 @@ __global__ void __launch_bounds__(256) k_nb_near(__grid_constant__ const NBArgs<
   const Blk bk = blk<B>(bm);
   const NBArgs<float>& A = B ? *tab[bk.sys] : A0;
   Scalars* sc = A.sc;
-  if (nb_idle(A)) return;
-  __shared__ long long red[32 + 9 * 8];  // block_sum_i64: 32 results + 9 per warp
+  if (A.near_in_collect || nb_idle(A)) return;
+  __shared__ long long red[9 + 9 * 8];
   const unsigned n = sc->near_n[A.work];
   if (n > (unsigned)A.near_cap) {
-    // the pairs did not fit: record the need and abort the step, which the
-    // host repeats with a larger buffer (as for the Verlet-list storage)
     __syncthreads();  // every thread has read the count
-    if (threadIdx.x == 0) {
-      sc->need_near[A.work] = (int)n;
-      sc->near_n[A.work] = 0u;
-      sc->abort = 1;
-      sc->skip = 1;
-    }
+    if (threadIdx.x == 0) near_overflow(sc, A.work, n);
     return;
   }
   const float ux = (float)(sc->box[0] * 0x1p-32), uy = (float)(sc->box[1] * 0x1p-32), uz = (float)(sc->box[2] * 0x1p-32);
@@ -2175,51 +2218,20 @@ __global__ void __launch_bounds__(256) k_nb_near(__grid_constant__ const NBArgs<
   long long acc[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
   for (unsigned k = threadIdx.x; k < n; k += blockDim.x) {
     const int4 nk = A.near[k];
-    const int s = nk.x, t = nk.y;
-    const int4 pi = A.posq[s], pj = A.posq[t];
-    const float d0 = (float)(int)((unsigned)pi.x - (unsigned)pj.x) * ux;
-    const float d1 = (float)(int)((unsigned)pi.y - (unsigned)pj.y) * uy;
-    const float d2 = (float)(int)((unsigned)pi.z - (unsigned)pj.z) * uz;
-    const float r2 = __fmaf_rn(d2, d2, __fmaf_rn(d1, d1, d0 * d0));
-    if (!inside_as_fp64(A, sc, nk.z, nk.w, r2)) continue;
-    const int ti = pi.w & 0xffff, li = pi.w >> 16, tj = pj.w & 0xffff, lj = pj.w >> 16;
-    const int4 pt = A.ptab[ti * A.ntype + tj];
-    if (!pt.w) { err |= EB_MISSING_TABLE; continue; }
-    const float r = r2 * rsqrtf(r2);
-    const float ib = __int_as_float(pt.z);
-    const int ni = (int)(r * ib);
-    if (ni > pt.y) { err |= EB_TABLE_RANGE; continue; }
-    const int row = pt.x + ni;
-    const float alpha = (r - A.tx[row]) * ib;
-    const float2 a0 = ((const float2*)A.tfp)[row], a1 = ((const float2*)A.tfp)[row + 1];
-    const float fij = __fmaf_rn(a1.x - a0.x, alpha, a0.x);
-    const float vij = __fmaf_rn(a1.y - a0.y, alpha, a0.y);
-    if (!(fabsf(fij) * r < 0.99f * kFixMax)) { err |= EB_FIXED; continue; }
-    const float fx = fij * d0, fy = fij * d1, fz = fij * d2;
-    const long long qx = __float2ll_rn(fx * kFixScale), qy = __float2ll_rn(fy * kFixScale),
-                    qz = __float2ll_rn(fz * kFixScale);
-    unsigned long long* fsi = (unsigned long long*)A.fsort + fs_at(s);
-    unsigned long long* fsj = (unsigned long long*)A.fsort + fs_at(t);
-    atomicAdd(fsi, (unsigned long long)qx);
-    atomicAdd(fsi + 32, (unsigned long long)qy);
-    atomicAdd(fsi + 64, (unsigned long long)qz);
-    atomicAdd(fsj, (unsigned long long)(-qx));
-    atomicAdd(fsj + 32, (unsigned long long)(-qy));
-    atomicAdd(fsj + 64, (unsigned long long)(-qz));
-    const bool lab3 = li == 3 || lj == 3;
-    const long long qe = fixq<24>(vij, err);
-    if (li == 1) acc[0] += qe;
-    if (li == 2 && lj == 2) acc[1] += qe;
-    if (li != 1 && lab3) acc[2] += qe;
-    acc[3] += fixq<24>(fx * d0, err);
-    acc[4] += fixq<24>(fy * d1, err);
-    acc[5] += fixq<24>(fz * d2, err);
-    acc[6] += fixq<24>(fy * d0, err);
-    acc[7] += fixq<24>(fz * d0, err);
-    acc[8] += fixq<24>(fz * d1, err);
+    long long f[3], e[9];
+    if (!near_pair(A, nk, ux, uy, uz, f, e, err)) continue;
+    unsigned long long* fsi = (unsigned long long*)A.fsort + fs_at(nk.x);
+    unsigned long long* fsj = (unsigned long long*)A.fsort + fs_at(nk.y);
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+      atomicAdd(fsi + 32 * c, (unsigned long long)f[c]);
+      atomicAdd(fsj + 32 * c, (unsigned long long)(-f[c]));
+    }
+#pragma unroll
+    for (int c = 0; c < 9; ++c) acc[c] += e[c];
   }
   if (err) atomicOr(&sc->err, err);
-  block_sum_i64<9>(acc, red);
+  block_sums<9>(acc, red);
   if (threadIdx.x < 9 && red[threadIdx.x] != 0)
     atomicAdd(&sc->nbacc[A.work][threadIdx.x], (unsigned long long)red[threadIdx.x]);
   __syncthreads();
@@ -2240,10 +2252,15 @@ struct CollectArgs {
   typename Prec<R>::acc_t* fsort;
   typename Prec<R>::acc_t* fnb;  // (3,NITEMS) global order
   typename Prec<R>::acc_t* mtsf; // [3][n][3] by A
+  // FP32 path, lists of one slot per thread: the list's nonbonded arguments on
+  // the device, whose pairs at the cutoff this kernel takes along; null where
+  // k_nb_near has done them
+  const NBArgs<float>* nb;
+  int work;
 };
 
 template <typename R, bool B>
-__global__ void k_nb_collect(__grid_constant__ const CollectArgs<R> C0, const CollectArgs<R>* const* tab,
+__global__ void __launch_bounds__(256, 5) k_nb_collect(__grid_constant__ const CollectArgs<R> C0, const CollectArgs<R>* const* tab,
                              const BlockMap bm) {
   using P = Prec<R>;
   pdl_wait();
@@ -2253,6 +2270,47 @@ __global__ void k_nb_collect(__grid_constant__ const CollectArgs<R> C0, const Co
   if (sc->skip) return;
   const int m = sc->mts_m;
   const bool explicit_step = !C.mts || (m >= 1 && m <= 3);
+  // The pairs at the cutoff (a few per 10,000 particles): every block goes
+  // through the list of them and computes those with a slot of its own, so
+  // that no launch of its own stands between the nonbonded kernel and this
+  // one.  k_finalize clears the count.
+  __shared__ unsigned long long s_near[3][256];
+  unsigned near_n = 0;
+  if constexpr (sizeof(R) == 4) {
+    if (C.nb && explicit_step) near_n = sc->near_n[C.work];
+    if (near_n > 0) {
+      const NBArgs<float>& A = *C.nb;
+      if (near_n > (unsigned)A.near_cap) {
+        __syncthreads();  // every thread of the block has read the count
+        if (bk.b == 0 && threadIdx.x == 0) near_overflow(sc, C.work, near_n);
+        return;
+      }
+#pragma unroll
+      for (int c = 0; c < 3; ++c) s_near[c][threadIdx.x] = 0ull;
+      __syncthreads();
+      const float ux = (float)(sc->box[0] * 0x1p-32), uy = (float)(sc->box[1] * 0x1p-32),
+                  uz = (float)(sc->box[2] * 0x1p-32);
+      for (unsigned k = threadIdx.x; k < near_n; k += blockDim.x) {
+        const int4 nk = A.near[k];
+        const bool own_i = (nk.x >> 8) == bk.b, own_j = (nk.y >> 8) == bk.b;
+        if (!own_i && !own_j) continue;
+        long long f[3], e[9];
+        unsigned err = 0;
+        if (near_pair(A, nk, ux, uy, uz, f, e, err)) {
+#pragma unroll
+          for (int c = 0; c < 3; ++c) {
+            if (own_i) atomicAdd(&s_near[c][nk.x & 255], (unsigned long long)f[c]);
+            if (own_j) atomicAdd(&s_near[c][nk.y & 255], (unsigned long long)(-f[c]));
+          }
+          if (own_i)
+            for (int c = 0; c < 9; ++c)
+              if (e[c] != 0) atomicAdd(&sc->nbacc[C.work][c], (unsigned long long)e[c]);
+        }
+        if (own_i && err) atomicOr(&sc->err, err);
+      }
+      __syncthreads();
+    }
+  }
   for (int s = bk.b * blockDim.x + threadIdx.x; s < C.n; s += bk.g * blockDim.x) {
     const int a = C.sorted[s];
     const int gi = C.idx[a];
@@ -2262,6 +2320,9 @@ __global__ void k_nb_collect(__grid_constant__ const CollectArgs<R> C0, const Co
       typename P::acc_t v[3];
 #pragma unroll
       for (int c = 0; c < 3; ++c) v[c] = C.fsort[fs_at(s) + 32 * c];
+      if (sizeof(R) == 4 && near_n > 0)
+#pragma unroll
+        for (int c = 0; c < 3; ++c) v[c] += (typename P::acc_t)s_near[c][threadIdx.x];
 #pragma unroll
       for (int c = 0; c < 3; ++c) {
         C.fnb[3 * (size_t)gi + c] = v[c];
@@ -2382,7 +2443,7 @@ __global__ void __launch_bounds__(256) k_bonded(__grid_constant__ const BondedAr
   const Blk bk = blk<BA>(bm);
   const BondedArgs<A>& B = BA ? *tab[bk.sys] : B0;
   Scalars* sc = B.sc;
-  __shared__ double red[12 * 8];
+  __shared__ double red[12 + 12 * 8];
   double acc[12];
 #pragma unroll
   for (int k = 0; k < 12; ++k) acc[k] = 0.0;
@@ -2622,10 +2683,8 @@ __global__ void __launch_bounds__(256) k_bonded(__grid_constant__ const BondedAr
     }
   }
   if (overext) atomicAdd(&sc->bond_overext, overext);
-  double out[12];
-  block_sum<12>(acc, red, out);
-  if (threadIdx.x == 0)
-    for (int k = 0; k < 12; ++k) B.part[k * B.part_stride + bk.b] = out[k];
+  block_sums<12>(acc, red);
+  if (threadIdx.x < 12) B.part[threadIdx.x * B.part_stride + bk.b] = red[threadIdx.x];
 }
 
 // ------------------------------------------------------------ integration
@@ -2652,7 +2711,7 @@ struct MoveArgs {
 // bonded forces are folded into the nonbonded array (fnb becomes the total
 // force FXYZ of the step) and cleared for the next step.
 template <typename R, bool B>
-__global__ void __launch_bounds__(256) k_move(__grid_constant__ const MoveArgs<R> M0, const MoveArgs<R>* const* tab,
+__global__ void __launch_bounds__(256, 3) k_move(__grid_constant__ const MoveArgs<R> M0, const MoveArgs<R>* const* tab,
                                               const BlockMap bm) {
   using P = Prec<R>;
   pdl_wait();
@@ -2660,7 +2719,7 @@ __global__ void __launch_bounds__(256) k_move(__grid_constant__ const MoveArgs<R
   const Blk bk = blk<B>(bm);
   const MoveArgs<R>& M = B ? *tab[bk.sys] : M0;
   Scalars* sc = M.sc;
-  __shared__ double red[18 * 8];
+  __shared__ double red[18 + 18 * 8];
   double acc[18];
 #pragma unroll
   for (int k = 0; k < 18; ++k) acc[k] = 0.0;
@@ -2706,31 +2765,30 @@ __global__ void __launch_bounds__(256) k_move(__grid_constant__ const MoveArgs<R
       M.S[3 * (size_t)i + c] = s[c] + M.dt * vn;
       vt[c] = 0.5 * (vn + v[c]);
     }
-    const int o = 6 * cls;
-    acc[o + 0] += m * vt[0] * vt[0];
-    acc[o + 1] += m * vt[1] * vt[1];
-    acc[o + 2] += m * vt[2] * vt[2];
-    acc[o + 3] += m * vt[0] * vt[1];
-    acc[o + 4] += m * vt[0] * vt[2];
-    acc[o + 5] += m * vt[1] * vt[2];
+    // both classes' sums, the other class's term zero (an index by class would
+    // put the sums into local memory)
+    const double ma = cls ? 0.0 : m, mb = cls ? m : 0.0;
+#pragma unroll
+    for (int k = 0; k < 6; ++k) {
+      const double x = vt[k < 3 ? k : (k < 5 ? 0 : 1)], y = vt[k < 3 ? k : (k == 3 ? 1 : 2)];
+      acc[k] += ma * x * y;
+      acc[6 + k] += mb * x * y;
+    }
   }
-  double out[18];
-  block_sum<18>(acc, red, out);
-  if (threadIdx.x == 0)
-    for (int k = 0; k < 18; ++k) M.part[k * M.part_stride + bk.b] = out[k];
+  block_sums<18>(acc, red);
+  if (threadIdx.x < 18) M.part[threadIdx.x * M.part_stride + bk.b] = red[threadIdx.x];
 }
 
 // Initial kinetic energies (main.F90:179-195).  Partials: EK atoms, EK beads.
 __global__ void k_kinetic(int natoms, const double* V, const int* tbits, const double* mass, double* part, int stride) {
-  __shared__ double red[2 * 8];
+  __shared__ double red[2 + 2 * 8];
   double acc[2] = {0.0, 0.0};
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < natoms; i += gridDim.x * blockDim.x) {
     const double* v = V + 3 * (size_t)i;
     acc[(tbits[i] >> 16) == 2 ? 1 : 0] += mass[i] * ((v[0] * v[0] + v[1] * v[1]) + v[2] * v[2]);
   }
-  double out[2];
-  block_sum<2>(acc, red, out);
-  if (threadIdx.x == 0) { part[blockIdx.x] = out[0]; part[stride + blockIdx.x] = out[1]; }
+  block_sums<2>(acc, red);
+  if (threadIdx.x < 2) part[threadIdx.x * stride + blockIdx.x] = red[threadIdx.x];
 }
 
 struct MomArgs {
@@ -2751,14 +2809,12 @@ __global__ void k_mom_sum(__grid_constant__ const MomArgs A0, const MomArgs* con
   const MomArgs& A = B ? *tab[bk.sys] : A0;
   const Scalars* sc = A.sc;
   if (sc->skip || sc->step % A.halt_drift != 0) return;
-  __shared__ double red[3 * 8];
+  __shared__ double red[3 + 3 * 8];
   double acc[3] = {0.0, 0.0, 0.0};
   for (int i = bk.b * blockDim.x + threadIdx.x; i < A.natoms; i += bk.g * blockDim.x)
     for (int c = 0; c < 3; ++c) acc[c] += A.V[3 * (size_t)i + c] * A.mass[i];
-  double out[3];
-  block_sum<3>(acc, red, out);
-  if (threadIdx.x == 0)
-    for (int c = 0; c < 3; ++c) A.part[c * A.nblocks + bk.b] = out[c];
+  block_sums<3>(acc, red);
+  if (threadIdx.x < 3) A.part[threadIdx.x * A.nblocks + bk.b] = red[threadIdx.x];
 }
 
 template <bool B>
@@ -2839,6 +2895,18 @@ __global__ void k_finalize(__grid_constant__ const FinalArgs F0, const FinalArgs
   __shared__ double q[64];
   if (sc->skip) return;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
+  // what warp 0 needs of the scalars after the sums, on its way meanwhile
+  const int m = sc->mts_m, step = sc->step, stop_at = sc->stop_at, iavp = sc->iavp, ring_base = sc->ring_base;
+  const unsigned err = sc->err;
+  const unsigned long long overext = sc->bond_overext, clamps = sc->cell_clamps;
+  double box[3];
+  for (int c = 0; c < 3; ++c) box[c] = sc->box[c];
+  const double prev = ((const double*)&sc->obs)[lane];
+  double h3 = 0.0, h1 = 0.0;  // MTS history of bead sum `lane`: V_NB(1..3), PT11..PT23
+  if (F.mts && lane < 9) {
+    h3 = lane < 3 ? sc->mts_vnb[2][lane] : sc->mts_pt[lane - 3][2];
+    h1 = lane < 3 ? sc->mts_vnb[0][lane] : sc->mts_pt[lane - 3][0];
+  }
   // q[0..8] atom NB, q[9..17] bead NB, q[18..29] bonded, q[30..47] move
   if (threadIdx.x < 18) {
     unsigned long long* p = &sc->nbacc[threadIdx.x / 9][threadIdx.x % 9];
@@ -2853,79 +2921,91 @@ __global__ void k_finalize(__grid_constant__ const FinalArgs F0, const FinalArgs
     if (lane == 0) q[k] = v;
   }
   __syncthreads();
-  if (threadIdx.x) return;
-  ObsD& o = sc->obs;
-  double bead_v[3], bead_pt[6];
-  for (int c = 0; c < 3; ++c) bead_v[c] = q[9 + c];
-  for (int c = 0; c < 6; ++c) bead_pt[c] = q[12 + c];
-  const int m = sc->mts_m;
-  if (F.mts) {
-    if (m >= 1 && m <= 3) {
-      for (int c = 0; c < 3; ++c) sc->mts_vnb[m - 1][c] = bead_v[c];
-      for (int c = 0; c < 5; ++c) sc->mts_pt[c][m - 1] = bead_pt[c];  // PT23 is not saved (MTS_LOOP.f90:193-199)
-    } else {
-      const double coef = (double)(m - 3) * 0.5;
-      for (int c = 0; c < 3; ++c) bead_v[c] = sc->mts_vnb[2][c] + coef * (sc->mts_vnb[2][c] - sc->mts_vnb[0][c]);
-      for (int c = 0; c < 6; ++c) bead_pt[c] = sc->mts_pt[c][2] + coef * (sc->mts_pt[c][2] - sc->mts_pt[c][0]);
+  if (warp) return;
+  // lane c < 9: sum c of both lists, 0..2 the energies and 3..8 the virial
+  double sum = 0.0;
+  if (lane < 9) {
+    double bead = q[9 + lane];
+    if (F.mts) {
+      if (m >= 1 && m <= 3) {
+        // PT23 is not saved (MTS_LOOP.f90:193-199)
+        if (lane < 3) sc->mts_vnb[m - 1][lane] = bead;
+        else if (lane < 8) sc->mts_pt[lane - 3][m - 1] = bead;
+      } else {
+        bead = h3 + (double)(m - 3) * 0.5 * (h3 - h1);
+      }
     }
+    sum = q[lane] + bead;
+    if (lane >= 3) sum = sum + q[42 + lane - 3];
   }
-  for (int c = 0; c < 3; ++c) {
-    o.v_nb[c] = q[c] + bead_v[c];
-    o.v_bond[c] = q[18 + c];
-    o.v_angle[c] = q[21 + c];
-    o.v_torsion[c] = q[24 + c];
-    o.v_oop[c] = q[27 + c];
-  }
-  double pt[6];
-  for (int c = 0; c < 6; ++c) pt[c] = q[3 + c] + bead_pt[c] + q[42 + c];
+  double ek[2] = {0.0, 0.0}, temp[3] = {0.0, 0.0, 0.0};
   if (F.move) {
     // MOVE.F90:90-115
-    for (int c = 0; c < 6; ++c) pt[c] += q[30 + c] + q[36 + c];
-    o.ek[0] = 0.5 * (q[30] + q[31] + q[32]);
-    o.ek[1] = 0.5 * (q[36] + q[37] + q[38]);
-    o.temp = (o.ek[0] + o.ek[1]) * F.mktemp;
-    o.temp_atom = o.ek[0] * F.mktemp_atom;
-    o.temp_bead = o.ek[1] * F.mktemp_bead;
-    sc->temp_atom = o.temp_atom;
-    sc->temp_bead = o.temp_bead;
-    const double vol = sc->box[0] * sc->box[1] * sc->box[2];
-    for (int c = 0; c < 6; ++c) pt[c] /= vol;
-    if (F.ensemble == 1 || F.ensemble == 2) {  // MOVE.F90:32-38, for the next step
-      sc->lam[0] = sqrt(1.0 + F.fac * ((F.temp_in / o.temp_atom) - 1.0));
-      sc->lam[1] = sqrt(1.0 + F.fac * ((F.temp_in / o.temp_bead) - 1.0));
+    if (lane >= 3 && lane < 9) {
+      sum += q[30 + lane - 3] + q[36 + lane - 3];
+      sum /= box[0] * box[1] * box[2];
+    }
+    ek[0] = 0.5 * (q[30] + q[31] + q[32]);
+    ek[1] = 0.5 * (q[36] + q[37] + q[38]);
+    temp[0] = (ek[0] + ek[1]) * F.mktemp;
+    temp[1] = ek[0] * F.mktemp_atom;
+    temp[2] = ek[1] * F.mktemp_bead;
+    if (lane < 2) {
+      const double t = lane == 0 ? temp[1] : temp[2];
+      (lane == 0 ? sc->temp_atom : sc->temp_bead) = t;
+      if (F.ensemble == 1 || F.ensemble == 2)  // MOVE.F90:32-38, for the next step
+        sc->lam[lane] = sqrt(1.0 + F.fac * ((F.temp_in / t) - 1.0));
     }
     if (F.ensemble == 2) {  // SCALEBP.f90:18-41
-      sc->iavp = sc->iavp + 1;
-      if (sc->iavp > 10) sc->iavp -= 10;
-      sc->sp[sc->iavp - 1] = (pt[0] + pt[1] + pt[2]) / 3.0;
-      if (sc->step % 10 == 0) {
+      const double p3 = __shfl_sync(0xffffffffu, sum, 3), p4 = __shfl_sync(0xffffffffu, sum, 4),
+                   p5 = __shfl_sync(0xffffffffu, sum, 5);
+      int iv = iavp + 1;
+      if (iv > 10) iv -= 10;
+      const double now = (p3 + p4 + p5) / 3.0;
+      if (lane == 0) {
+        sc->iavp = iv;
+        sc->sp[iv - 1] = now;
+      }
+      if (step % 10 == 0) {
         double avp = 0.0;
-        for (int i = 0; i < 10; ++i) avp += sc->sp[i];
+        for (int i = 0; i < 10; ++i) avp += i == iv - 1 ? now : sc->sp[i];
         const double p = avp / 10.0;
         const double miu = pow(1.0 + (p - F.pressure) * F.pfac, 1.0 / 3.0);
-        sc->miu = miu;
-        for (int c = 0; c < 3; ++c) {
-          sc->box[c] *= miu;
-          sc->boxinv[c] = 1.0 / sc->box[c];
-          sc->box2[c] = sc->box[c] / 2.0;
-          sc->boxf[c] = (float)sc->box[c];
-          sc->boxinvf[c] = 1.0f / sc->boxf[c];
-          sc->box2f[c] = sc->boxf[c] / 2.0f;
+        for (int c = 0; c < 3; ++c) box[c] *= miu;
+        if (lane == 0) sc->miu = miu;
+        if (lane < 3) {
+          const double b = lane == 0 ? box[0] : (lane == 1 ? box[1] : box[2]);
+          sc->box[lane] = b;
+          sc->boxinv[lane] = 1.0 / b;
+          sc->box2[lane] = b / 2.0;
+          const float bf = (float)b;
+          sc->boxf[lane] = bf;
+          sc->boxinvf[lane] = 1.0f / bf;
+          sc->box2f[lane] = bf / 2.0f;
         }
       }
     }
   }
-  sc->done = sc->step >= sc->stop_at;
-  for (int c = 0; c < 6; ++c) o.pt[c] = pt[c];
-  for (int c = 0; c < 3; ++c) o.box[c] = sc->box[c];
-  o.bond_overext = (long long)sc->bond_overext;
-  o.cell_clamps = (long long)sc->cell_clamps;
-  o.step = sc->step;
-  o.status = (int)sc->err;
-  if (F.ring) {
-    int slot = sc->step - sc->ring_base;
-    if (slot >= 0 && slot < F.ring_cap) F.ring[slot] = o;
-  }
+  // the observables, one 8-byte field per lane (a force stage keeps the
+  // kinetic part of the step before)
+  __shared__ double ob[32];
+  ob[lane] = prev;
+  __syncwarp();
+  if (F.move && lane < 5) ob[lane] = lane < 2 ? ek[lane & 1] : temp[lane - 2];
+  if (lane < 3) ob[5 + lane] = sum;
+  if (lane < 12) ob[8 + lane] = q[18 + lane];
+  if (lane >= 3 && lane < 9) ob[20 + lane - 3] = sum;
+  if (lane < 3) ob[26 + lane] = lane == 0 ? box[0] : (lane == 1 ? box[1] : box[2]);
+  if (lane == 29) ob[29] = __longlong_as_double((long long)overext);
+  if (lane == 30) ob[30] = __longlong_as_double((long long)clamps);
+  if (lane == 31) ob[31] = __longlong_as_double((long long)(((unsigned long long)err << 32) | (unsigned)step));
+  __syncwarp();
+  static_assert(sizeof(ObsD) == 32 * sizeof(double), "one field per lane");
+  ((double*)&sc->obs)[lane] = ob[lane];
+  if (lane == 0) sc->done = step >= stop_at;
+  if (lane < 2) sc->near_n[lane] = 0u;
+  const int slot = step - ring_base;
+  if (F.ring && slot >= 0 && slot < F.ring_cap) ((double*)&F.ring[slot])[lane] = ob[lane];
 }
 
 // Step counter, observable ring base and step limit of the next run.

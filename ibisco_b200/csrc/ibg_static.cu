@@ -83,7 +83,7 @@ __device__ __forceinline__ long long fixq(float v, unsigned* err) {
 constexpr int kWideLists = 45000;
 template <int T>
 __global__ void __launch_bounds__(256) k_static_pairs(StaticArgs a) {
-  __shared__ double red[9 * 8];
+  __shared__ double red[9 + 9 * 8];
   double acc[9];
 #pragma unroll
   for (int k = 0; k < 9; ++k) acc[k] = 0.0;
@@ -178,10 +178,8 @@ __global__ void __launch_bounds__(256) k_static_pairs(StaticArgs a) {
       atomicAdd(&a.f[3 * (long long)i + 2], (unsigned long long)f2);
     }
   }
-  double out[9];
-  ibg::block_sum<9>(acc, red, out);
-  if (threadIdx.x == 0)
-    for (int k = 0; k < 9; ++k) a.part[9 * blockIdx.x + k] = out[k];
+  ibg::block_sums<9>(acc, red);
+  if (threadIdx.x < 9) a.part[9 * blockIdx.x + threadIdx.x] = red[threadIdx.x];
 }
 
 // Forces to FP64 (3,NITEMS) and the block partials to V_NB(1..3), PT11, PT22,
