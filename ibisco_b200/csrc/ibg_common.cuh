@@ -70,6 +70,7 @@ struct Scalars {
   int done;           // stop_at reached: set by the last step's k_finalize
   int need_rows[2];   // rows of 32 entries a slice of each list needed
   int rows_max[2];    // most rows of any slice of each list, at its last build
+  int cell_max[2];    // most particles of any cell of each list, at its last build
   unsigned work[4];   // dynamic work counters: nonbonded atom/bead, list build atom/bead
   unsigned near_n[2];  // pairs at the cutoff left by the FP32 nonbonded kernel, per list
   int need_near[2];    // pairs at the cutoff a list needed room for (the step is repeated)

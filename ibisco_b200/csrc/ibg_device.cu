@@ -37,10 +37,12 @@ using namespace ibg;
 
 namespace {
 
-// Particles per SM from which a list is built with a thread per particle:
-// 64 resident warps of 32 particles each, twice over.  Measured: the
-// 2,000,000-bead melt builds in 1.97 ms a thread per particle against 3.0 ms a
-// warp per particle; the 40,000-bead melt takes 225 us against 140 us.
+// Particles per SM from which a list is built with a thread per particle: 64
+// resident warps of 32 particles each, twice over.  Whole rebuild (cell sort
+// and lists), units of a cell's particles against a thread per particle: the
+// 2,000,000-bead melt 2.72 ms against 2.11, a 160,000-bead one 261 us against
+// 283, the 40,000-bead melt 105 against 165, the hybrid melt (two lists) 252
+// against 579.
 constexpr long long kThreadBuildMin = 2LL * 64 * 32;
 
 struct CudaError {
@@ -119,11 +121,11 @@ struct DevList {
   int form = 0;
   int cell_cap = 0, nslices = 0;
   int w_cap = 0;  // rows of 32 list entries per slice
-  int *idx = nullptr, *cell_of = nullptr, *cell_count = nullptr, *cell_start = nullptr, *cell_fill = nullptr;
-  int *sorted = nullptr, *sorted_new = nullptr, *slot_of = nullptr, *slot_of_new = nullptr;
+  int *idx = nullptr, *cell_of = nullptr, *cell_count = nullptr, *cell_start = nullptr;
+  int *sorted = nullptr, *slot_of = nullptr, *place = nullptr, *cells = nullptr;
   int *counts = nullptr, *slice_w = nullptr, *entries = nullptr;
-  void *pos4 = nullptr, *pos4_new = nullptr, *fsort = nullptr, *mtsf = nullptr;
-  int4 *posq = nullptr, *posq_new = nullptr;  // FP32 path: positions as box fractions
+  void *pos4 = nullptr, *fsort = nullptr, *mtsf = nullptr;
+  int4* posq = nullptr;  // FP32 path: positions as box fractions
   int4* near = nullptr;                       // FP32 path: pairs at the cutoff (k_nb_near)
   int near_cap = 0;
   size_t pos_bytes = 0;
@@ -197,7 +199,7 @@ struct ibg_ctx {
   SysArgs<float> af;
   SysArgs<double> ad;
   void* dargs = nullptr;  // device copy of af or ad
-  int g_list[2] = {1, 1}, g_regrid[2] = {1, 1}, g_build[2] = {1, 1}, g_dist = 1;
+  int g_list[2] = {1, 1}, g_build[2] = {1, 1}, g_dist = 1;
   int nb_blocks_per_sm = 0;  // tuning: resident nonbonded blocks per SM (0: all that fit)
   int nb_chunk = 0;          // tuning (FP32): 256ths of the units taken dynamically after the block ranges (0: all, per warp)
   int nb_rows = 16;          // tuning: list rows per nonbonded work unit (8 or 16)
@@ -320,20 +322,18 @@ void build_list(ibg_ctx* c, const ibg_desc* d, int which) {
   L.idx = dupload(idx, o);
   L.cell_of = dalloc<int>(L.n, o);
   L.sorted = dalloc<int>(L.n, o);
-  L.sorted_new = dalloc<int>(L.n, o);
+  L.place = dalloc<int>(L.n, o);
+  L.cells = dalloc<int>(L.n, o);
   std::vector<int> ident(L.n);
   for (int a = 0; a < L.n; ++a) ident[a] = a;
   L.slot_of = dupload(ident, o);
   CK(cudaMemcpy(L.sorted, ident.data(), sizeof(int) * L.n, cudaMemcpyHostToDevice));
-  L.slot_of_new = dalloc<int>(L.n, o);
   L.counts = dalloc<int>(L.n, o);
   L.slice_w = dalloc<int>(L.nslices, o);
   L.pos_bytes = possize(c) * L.n;
   L.pos4 = dalloc<unsigned char>(L.pos_bytes, o);
-  L.pos4_new = dalloc<unsigned char>(L.pos_bytes, o);
   if (c->prec == IBG_PREC_FP32_FIXED) {
     L.posq = dalloc<int4>(L.n, o);
-    L.posq_new = dalloc<int4>(L.n, o);
     // about 16 pairs a step sit this close to the cutoff on 40,000 beads
     L.near_cap = std::max(4096, L.n / 32);
     L.near = dalloc<int4>(L.near_cap, o);
@@ -458,7 +458,6 @@ void alloc_cells(ibg_ctx* c, DevList& L, const float* box) {
   L.cell_cap = (int)ncap;
   L.cell_count = dalloc_now<int>(ncap, o);
   L.cell_start = dalloc_now<int>(ncap + 1, o);
-  L.cell_fill = dalloc_now<int>(ncap, o);
 }
 
 int grid_for(ibg_ctx* c, long long work, int per_sm = 8) {
@@ -531,10 +530,8 @@ void make_args(ibg_ctx* c) {
     a.nslices = L.nslices;
     a.rlist = L.rlist; a.rlistsq = L.rlistsq; a.rlistd = (double)L.rlist; a.rlistsqd = (double)L.rlist * (double)L.rlist;
     a.idx = L.idx; a.cell_of = L.cell_of; a.cell_count = L.cell_count; a.cell_start = L.cell_start;
-    a.cell_fill = L.cell_fill;
-    a.sorted = L.sorted; a.sorted_new = L.sorted_new; a.slot_of = L.slot_of; a.slot_of_new = L.slot_of_new;
-    a.gslot = c->gslot; a.pos4 = L.pos4; a.pos4_new = L.pos4_new;
-    a.posq = L.posq; a.posq_new = L.posq_new;
+    a.place = L.place; a.cells = L.cells; a.sorted = L.sorted; a.slot_of = L.slot_of;
+    a.gslot = c->gslot; a.pos4 = L.pos4; a.posq = L.posq; a.S = c->S; a.tbits = c->tbits;
     a.counts = L.counts; a.slice_w = L.slice_w; a.entries = L.entries; a.w_cap = L.w_cap;
     a.rgroupsq = L.rgroupsq;
     a.excl_n = c->excl_n; a.excl = c->excl;
@@ -653,21 +650,17 @@ void enq_rebuild(ibg_ctx* c, DevList& L, int always) {
   if (!L.present) return;
   const ListArgs& a = args<R>(c).list[L.which];
   const int w = L.which, gn = c->g_list[w];
-  // the first launch may follow a memset (ibg_set_state): an ordinary one;
-  // the rest follow a kernel of the chain
+  // in a step the first launch follows k_positions or the other list's build;
+  // in ibg_set_state it may follow a memset: an ordinary launch there
   using LA = const ListArgs* const*;
-  k_regrid<R, false><<<c->g_regrid[w], 256, 0, c->st>>>(a, nullptr, kOne, always);
+  launch_on(c->st, c->pdl && !c->timing && !always, k_cell_assign<R, false>, gn, 256, 0, a, (LA)nullptr, kOne, always);
   ++c->launches;
-  launch_pdl(c, k_cell_assign<R, false>, gn, 256, 0, a, (LA)nullptr, kOne, always);
   launch_pdl(c, k_scan_cells<false>, 1, 1024, 0, a, (LA)nullptr, kOne, always);
   launch_pdl(c, k_cell_fill<false>, gn, 256, 0, a, (LA)nullptr, kOne, always);
-  launch_pdl(c, k_cell_rank<false>, gn, 256, 0, a, (LA)nullptr, kOne, always);
-  launch_pdl(c, k_reslot<R, false>, gn, 256, 0, a, (LA)nullptr, kOne, always);
-  launch_pdl(c, k_slot_of<R, false>, gn, 256, 0, a, (LA)nullptr, kOne, always);
+  launch_pdl(c, k_cell_rank<R, false>, gn, 256, 0, a, (LA)nullptr, kOne, always);
   const int gl = c->g_build[w];
-  // a thread per particle once the list has enough particles to fill the GPU
-  // that way (twice the resident warps), a warp per particle below that;
-  // both give the same lists
+  // lists long enough to fill the GPU with a thread per particle: the thread
+  // build; both give the same lists (kThreadBuildMin)
   if (L.form == 1)
     launch_pdl(c, k_list_build_slices<false>, gl, 256, 0, a, (LA)nullptr, kOne, always);
   else if (L.n >= kThreadBuildMin * c->nsm)
@@ -1578,7 +1571,6 @@ std::vector<unsigned char> graph_key(const ibg_ctx* c) {
   };
   if (c->prec == IBG_PREC_FP32_FIXED) add(&c->af, sizeof(c->af));
   else add(&c->ad, sizeof(c->ad));
-  add(c->g_regrid, sizeof(c->g_regrid));
   return k;
 }
 
@@ -1619,7 +1611,6 @@ int ibg_set_state(ibg_ctx* c, const float* sxyz, const float* vxyz, const float*
       alloc_cells(c, L, box);
       CK(cudaMemsetAsync(L.fsort, 0, accsize(c) * fs_len(L.n), c->st));
       if (L.mtsf) CK(cudaMemsetAsync(L.mtsf, 0, accsize(c) * 9 * (size_t)L.n, c->st));
-      c->g_regrid[L.which] = grid_for(c, L.cell_cap, 2);
     }
     CK(cudaMemsetAsync(c->fnb, 0, accsize(c) * 3 * (size_t)c->nitems, c->st));
     CK(cudaMemsetAsync(c->fb, 0, accsize(c) * 3 * (size_t)c->nitems, c->st));
@@ -2015,7 +2006,7 @@ struct ibg_batch {
   void** t_move = nullptr;
   void** t_mom = nullptr;
   void** t_fin = nullptr;
-  BMap m_pos, m_regrid[2], m_list[2], m_scan[2], m_dist, m_bond, m_move, m_fin;
+  BMap m_pos, m_list[2], m_scan[2], m_dist, m_bond, m_move, m_fin;
   std::vector<NBGroup> lb[2];  // list build, by T (smem unused)
   std::vector<NBGroup> nb[2];  // nonbonded, by (T, smem)
   bool any_vs = false, any_list[2] = {false, false};
@@ -2087,8 +2078,6 @@ void batch_layout(ibg_batch* b) {
     for (size_t s = 0; s < n; ++s) b->any_list[w] |= b->sys[s]->L[w].present;
     for (size_t s = 0; s < n; ++s)
       b->any_near[w] |= b->prec == IBG_PREC_FP32_FIXED && b->sys[s]->L[w].present && !near_in_collect(b->sys[s], b->sys[s]->L[w]);
-    for (size_t s = 0; s < n; ++s) g[s] = b->sys[s]->L[w].present ? b->sys[s]->g_regrid[w] : 0;
-    b->m_regrid[w] = make_map(b, g);
     for (size_t s = 0; s < n; ++s) g[s] = b->sys[s]->L[w].present ? b->sys[s]->g_list[w] : 0;
     b->m_list[w] = make_map(b, g);
     for (size_t s = 0; s < n; ++s) g[s] = b->sys[s]->L[w].present ? 1 : 0;
@@ -2177,14 +2166,11 @@ void batch_enqueue(ibg_batch* b, unsigned v) {
       if (!b->any_list[w]) continue;
       const ListArgs* const* t = (const ListArgs* const*)b->t_list[w];
       const BMap& ml = b->m_list[w];
-      k_regrid<R, true><<<b->m_regrid[w].grid, 256, 0, st>>>(ListArgs{}, t, b->m_regrid[w].m(), 0);
       launch_on(st, true, k_cell_assign<R, true>, ml.grid, 256, 0, ListArgs{}, t, ml.m(), 0);
       launch_on(st, true, k_scan_cells<true>, b->m_scan[w].grid, 1024, 0, ListArgs{}, t, b->m_scan[w].m(), 0);
       launch_on(st, true, k_cell_fill<true>, ml.grid, 256, 0, ListArgs{}, t, ml.m(), 0);
-      launch_on(st, true, k_cell_rank<true>, ml.grid, 256, 0, ListArgs{}, t, ml.m(), 0);
-      launch_on(st, true, k_reslot<R, true>, ml.grid, 256, 0, ListArgs{}, t, ml.m(), 0);
-      launch_on(st, true, k_slot_of<R, true>, ml.grid, 256, 0, ListArgs{}, t, ml.m(), 0);
-      n += 7;
+      launch_on(st, true, k_cell_rank<R, true>, ml.grid, 256, 0, ListArgs{}, t, ml.m(), 0);
+      n += 4;
       for (const NBGroup& grp : b->lb[w]) {
         const BlockMap bm = grp.map.m();
         if (grp.form == 1)

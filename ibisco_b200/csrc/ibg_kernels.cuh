@@ -417,16 +417,15 @@ struct ListArgs {
   int* cell_of;      // [n] cell of list entry A
   int* cell_count;   // [cell_cap]
   int* cell_start;   // [cell_cap + 1]
-  int* cell_fill;    // [cell_cap]
+  int* place;        // [n] place of list entry A among its cell's entries
+  int* cells;        // [n] the cells' entries, one cell after another
   int* sorted;       // [n] slot -> A
-  int* sorted_new;   // [n]
   int* slot_of;      // [n] A -> slot
-  int* slot_of_new;  // [n]
   int* gslot;        // [NITEMS]
   void* pos4;        // [n]
-  void* pos4_new;    // [n]
   int4* posq;        // [n] FP32 path: fixed-point positions (box fractions), or null
-  int4* posq_new;    // [n]
+  const double* S;   // FP64 state (3,NITEMS)
+  const int* tbits;  // type | label<<16 per particle
   int* counts;       // [n] per slot
   int* slice_w;      // [nslices] rows of 32 entries used by each slice
   int* entries;      // list storage: slice g owns rows [g*w_cap, (g+1)*w_cap) of 32 entries
@@ -438,35 +437,16 @@ struct ListArgs {
 // List-rebuild kernels run when the step rebuilds its lists (or always, for
 // the rebuild of ibg_set_state) and the step is not skipped.
 //
+// Five launches: cells and counts, their scan, the cells' entries, their order
+// and new slots, the lists.  (They were eight; each costs ~4 us where the
+// system is small.)
+//
 // UPDATE_NEIGHBOURLIST.F90:14-48 / ALLOCATEVAR2.f90:19-42: cells per
-// dimension = INT(BOX/RLIST).  The grid also clears the cell counters.
-template <typename R, bool B>
-__global__ void k_regrid(__grid_constant__ const ListArgs L0, const ListArgs* const* tab, const BlockMap bm, int always) {
-  pdl_wait();
-  pdl_trigger();
-  const Blk bk = blk<B>(bm);
-  const ListArgs& L = B ? *tab[bk.sys] : L0;
-  Scalars* sc = L.sc;
-  if (sc->skip || !(always || sc->rebuild)) return;
-  for (int c = bk.b * blockDim.x + threadIdx.x; c < L.cell_cap; c += bk.g * blockDim.x) L.cell_count[c] = 0;
-  for (int g = bk.b * blockDim.x + threadIdx.x; g < L.nslices; g += bk.g * blockDim.x) L.slice_w[g] = 0;
-  if (threadIdx.x || bk.b) return;
-  sc->rows_max[L.which] = 0;
-  int nc[3];
-  for (int c = 0; c < 3; ++c) {
-    if (sizeof(R) == 4) nc[c] = fint(sc->boxf[c] / L.rlist);
-    else nc[c] = fint(sc->box[c] / L.rlistd);
-  }
-  bool bad = nc[0] < 3 || nc[1] < 3 || nc[2] < 3;
-  long long tot = (long long)nc[0] * nc[1] * nc[2];
-  if (bad) atomicOr(&sc->err, EB_CELL_GRID);
-  if (tot > L.cell_cap) atomicOr(&sc->err, EB_CAPACITY);
-  if (bad || tot > L.cell_cap) nc[0] = nc[1] = nc[2] = 1;
-  for (int c = 0; c < 3; ++c) sc->ncell[L.which][c] = nc[c];
-}
-
-// LINKS.f90:16-18.  A component equal to NCELL (coordinate at +L/2 after
-// rounding) would address a cell outside the grid; it is clamped and counted.
+// dimension = INT(BOX/RLIST), and LINKS.f90:16-18.  A component equal to NCELL
+// (coordinate at +L/2 after rounding) would address a cell outside the grid;
+// it is clamped and counted.  The cell counters are zero at the start (when
+// allocated, and again after k_cell_fill).  An entry's place among its cell's
+// entries, in no particular order yet, is what its count returned.
 template <typename R, bool B>
 __global__ void k_cell_assign(__grid_constant__ const ListArgs L0, const ListArgs* const* tab, const BlockMap bm, int always) {
   pdl_wait();
@@ -476,14 +456,25 @@ __global__ void k_cell_assign(__grid_constant__ const ListArgs L0, const ListArg
   const ListArgs& L = B ? *tab[bk.sys] : L0;
   Scalars* sc = L.sc;
   if (sc->skip || !(always || sc->rebuild)) return;
-  const int nx = sc->ncell[L.which][0], ny = sc->ncell[L.which][1], nz = sc->ncell[L.which][2];
   R b[3], bi[3], b2[3];
   box_of<R>(sc, b, bi, b2);
+  int nc[3];
+#pragma unroll
+  for (int c = 0; c < 3; ++c) nc[c] = fint(b[c] / (sizeof(R) == 4 ? (R)L.rlist : (R)L.rlistd));
+  const bool bad = nc[0] < 3 || nc[1] < 3 || nc[2] < 3;
+  const bool full = (long long)nc[0] * nc[1] * nc[2] > L.cell_cap;
+  if (bad || full) nc[0] = nc[1] = nc[2] = 1;
+  if (bk.b == 0 && threadIdx.x == 0) {
+    if (bad) atomicOr(&sc->err, EB_CELL_GRID);
+    if (full) atomicOr(&sc->err, EB_CAPACITY);
+    for (int c = 0; c < 3; ++c) sc->ncell[L.which][c] = nc[c];
+    sc->rows_max[L.which] = 0;
+  }
   const PT* pos = (const PT*)L.pos4;
   for (int a = bk.b * blockDim.x + threadIdx.x; a < L.n; a += bk.g * blockDim.x) {
     PT p = pos[L.slot_of[a]];
     R x[3] = {p.x, p.y, p.z};
-    int nc[3] = {nx, ny, nz}, k[3];
+    int k[3];
     int clamps = 0;
 #pragma unroll
     for (int c = 0; c < 3; ++c) {
@@ -492,14 +483,14 @@ __global__ void k_cell_assign(__grid_constant__ const ListArgs L0, const ListArg
       if (k[c] < 0) { k[c] = 0; ++clamps; }
     }
     if (clamps) atomicAdd(&sc->cell_clamps, (unsigned long long)clamps);
-    int cell = k[0] * nz * ny + k[1] * nz + k[2];
+    const int cell = (k[0] * nc[1] + k[1]) * nc[2] + k[2];
     L.cell_of[a] = cell;
-    atomicAdd(&L.cell_count[cell], 1);
+    L.place[a] = atomicAdd(&L.cell_count[cell], 1);
   }
 }
 
 // Exclusive scan of the cell counts by one block per system (cell_start has
-// cell_cap + 1 entries); clears the fill counters.
+// cell_cap + 1 entries).
 template <bool B>
 __global__ void k_scan_cells(__grid_constant__ const ListArgs L0, const ListArgs* const* tab, const BlockMap bm, int always) {
   pdl_wait();
@@ -510,7 +501,6 @@ __global__ void k_scan_cells(__grid_constant__ const ListArgs L0, const ListArgs
   if (sc->skip || !(always || sc->rebuild)) return;
   const int* in = L.cell_count;
   int* out = L.cell_start;
-  int* zero = L.cell_fill;
   const int m = L.cell_cap;
   __shared__ int wsum[32];
   const int t = threadIdx.x, T = blockDim.x, lane = t & 31, warp = t >> 5, nw = (T + 31) >> 5;
@@ -518,7 +508,7 @@ __global__ void k_scan_cells(__grid_constant__ const ListArgs L0, const ListArgs
   // the tile (read and written as int4 where the tile is whole), the tiles in
   // order with the running total carried from one to the next
   constexpr int V = 16;
-  int carry = 0;
+  int carry = 0, most = 0;
   for (int base = 0; base < m; base += V * T) {
     const int i0 = base + V * t;
     const bool whole = i0 + V <= m;
@@ -534,7 +524,10 @@ __global__ void k_scan_cells(__grid_constant__ const ListArgs L0, const ListArgs
       for (int j = 0; j < V; ++j) x[j] = i0 + j < m ? in[i0 + j] : 0;
     }
 #pragma unroll
-    for (int j = 0; j < V; ++j) s += x[j];
+    for (int j = 0; j < V; ++j) {
+      s += x[j];
+      most = max(most, x[j]);
+    }
     int v = s;  // inclusive scan of the threads' sums: warps, then warp totals
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
@@ -562,24 +555,31 @@ __global__ void k_scan_cells(__grid_constant__ const ListArgs L0, const ListArgs
     }
     if (whole) {
 #pragma unroll
-      for (int j = 0; j < V / 4; ++j) {
+      for (int j = 0; j < V / 4; ++j)
         ((int4*)(out + i0))[j] = make_int4(x[4 * j], x[4 * j + 1], x[4 * j + 2], x[4 * j + 3]);
-        ((int4*)(zero + i0))[j] = make_int4(0, 0, 0, 0);
-      }
     } else {
 #pragma unroll
       for (int j = 0; j < V; ++j)
-        if (i0 + j < m) {
-          out[i0 + j] = x[j];
-          zero[i0 + j] = 0;
-        }
+        if (i0 + j < m) out[i0 + j] = x[j];
     }
     carry += wsum[nw - 1];
     __syncthreads();  // wsum is rewritten by the next tile
   }
-  if (t == 0) out[m] = carry;
+  // the fullest cell (the list build's units)
+  __shared__ int s_most;
+  if (t == 0) s_most = 0;
+  __syncthreads();
+  most = __reduce_max_sync(0xffffffffu, most);
+  if (lane == 0) atomicMax(&s_most, most);
+  __syncthreads();
+  if (t == 0) {
+    out[m] = carry;
+    sc->cell_max[L.which] = s_most;
+  }
 }
 
+// The cells' entries side by side, and the cell counters (for the next
+// rebuild) and slice lengths (for this one's lists) cleared.
 template <bool B>
 __global__ void k_cell_fill(__grid_constant__ const ListArgs L0, const ListArgs* const* tab, const BlockMap bm, int always) {
   pdl_wait();
@@ -588,94 +588,51 @@ __global__ void k_cell_fill(__grid_constant__ const ListArgs L0, const ListArgs*
   const ListArgs& L = B ? *tab[bk.sys] : L0;
   Scalars* sc = L.sc;
   if (sc->skip || !(always || sc->rebuild)) return;
-  for (int a = bk.b * blockDim.x + threadIdx.x; a < L.n; a += bk.g * blockDim.x) {
-    int c = L.cell_of[a];
-    int s = L.cell_start[c] + atomicAdd(&L.cell_fill[c], 1);
-    L.sorted_new[s] = a;
-  }
+  const int t0 = bk.b * blockDim.x + threadIdx.x, nt = bk.g * blockDim.x;
+  for (int a = t0; a < L.n; a += nt) L.cells[L.cell_start[L.cell_of[a]] + L.place[a]] = a;
+  for (int c = t0; c < L.cell_cap; c += nt) L.cell_count[c] = 0;
+  for (int g = t0; g < L.nslices; g += nt) L.slice_w[g] = 0;
 }
 
 // Within a cell the reference's linked list visits entries by decreasing A
 // (LINKS.f90:19-20); slots are kept in increasing A so the list build can
-// walk them backwards.  k_cell_fill placed a cell's entries in arbitrary order
-// (atomics); here each entry finds its rank among its cell's entries.
-template <bool B>
+// walk them backwards.  Each entry finds its rank among its cell's entries,
+// and with it its new slot; its position goes there from the FP64 state, as
+// k_positions stored it in the old slot (a site's row holds the value in the
+// step's precision).
+template <typename R, bool B>
 __global__ void k_cell_rank(__grid_constant__ const ListArgs L0, const ListArgs* const* tab, const BlockMap bm, int always) {
   pdl_wait();
   pdl_trigger();
-  const Blk bk = blk<B>(bm);
-  const ListArgs& L = B ? *tab[bk.sys] : L0;
-  Scalars* sc = L.sc;
-  if (sc->skip || !(always || sc->rebuild)) return;
-  for (int s = bk.b * blockDim.x + threadIdx.x; s < L.n; s += bk.g * blockDim.x) {
-    const int a = L.sorted_new[s];
-    const int c = L.cell_of[a];
-    const int b = L.cell_start[c], e = L.cell_start[c + 1];
-    int rank = 0;
-    for (int k = b; k < e; ++k) rank += L.sorted_new[k] < a;
-    L.slot_of_new[b + rank] = a;  // scratch: the ordered cell segment
-  }
-}
-
-// New slot order: positions move to their new slots, and the slot of every
-// entry (and of its global particle) is updated.  Reads the ordered cells from
-// the scratch k_cell_rank wrote; writes the new order to sorted.
-template <typename R, bool B>
-__global__ void k_reslot(__grid_constant__ const ListArgs L0, const ListArgs* const* tab, const BlockMap bm, int always) {
-  pdl_wait();
-  pdl_trigger();
   using PT = typename Prec<R>::pos_t;
   const Blk bk = blk<B>(bm);
   const ListArgs& L = B ? *tab[bk.sys] : L0;
   Scalars* sc = L.sc;
   if (sc->skip || !(always || sc->rebuild)) return;
+  R b[3], bi[3], b2[3];
+  box_of<R>(sc, b, bi, b2);
+  const double boxinv[3] = {sc->boxinv[0], sc->boxinv[1], sc->boxinv[2]};
   for (int s = bk.b * blockDim.x + threadIdx.x; s < L.n; s += bk.g * blockDim.x) {
-    int a = L.slot_of_new[s];
-    ((PT*)L.pos4_new)[s] = ((const PT*)L.pos4)[L.slot_of[a]];
-    if (L.posq) L.posq_new[s] = L.posq[L.slot_of[a]];
-    L.sorted[s] = a;
-    L.gslot[L.idx[a]] = s * 2 + L.which;
+    const int a = L.cells[s];
+    const int c = L.cell_of[a], i = L.idx[a];
+    const int lo = L.cell_start[c], hi = L.cell_start[c + 1];
+    const double sd[3] = {L.S[3 * (size_t)i], L.S[3 * (size_t)i + 1], L.S[3 * (size_t)i + 2]};
+    const int tb = L.tbits[i];
+    int slot = lo;
+    for (int k = lo; k < hi; ++k) slot += L.cells[k] < a;
+    R r[3] = {(R)sd[0], (R)sd[1], (R)sd[2]};
+    fold3<R>(r, b2);
+    PT p;
+    p.x = r[0]; p.y = r[1]; p.z = r[2];
+    p.w = Prec<R>::tbits(tb);
+    ((PT*)L.pos4)[slot] = p;
+    if (L.posq) L.posq[slot] = box_fraction(sd, boxinv, tb);
+    L.sorted[slot] = a;
+    L.slot_of[a] = slot;
+    L.gslot[i] = slot * 2 + L.which;
   }
 }
 
-// slot_of from the new order, and the positions into their new slots (after
-// k_reslot).
-template <typename R, bool B>
-__global__ void k_slot_of(__grid_constant__ const ListArgs L0, const ListArgs* const* tab, const BlockMap bm, int always) {
-  pdl_wait();
-  pdl_trigger();
-  using PT = typename Prec<R>::pos_t;
-  const Blk bk = blk<B>(bm);
-  const ListArgs& L = B ? *tab[bk.sys] : L0;
-  Scalars* sc = L.sc;
-  if (sc->skip || !(always || sc->rebuild)) return;
-  for (int s = bk.b * blockDim.x + threadIdx.x; s < L.n; s += bk.g * blockDim.x) {
-    L.slot_of[L.sorted[s]] = s;
-    ((PT*)L.pos4)[s] = ((const PT*)L.pos4_new)[s];
-    if (L.posq) L.posq[s] = L.posq_new[s];
-  }
-}
-
-// NEW_NEIGHBOUR_WITHLIST.f90:34-123 for lists of up to a few hundred
-// thousand particles.  A block builds the lists of one cell's
-// particles at a time (cells taken dynamically).  The candidates of the cell --
-// its own slots, then the slots of the 13 cells of the MAPS.f90:39-51
-// stencil, each run by decreasing A -- are staged once in shared memory, in
-// that order, with their slot numbers; every particle of the cell then reads
-// them from there.  A warp builds one particle's list: its candidates are the
-// staged ones from just below its own slot to the end, which is the
-// reference's order (its own cell below it by decreasing A, then the stencil
-// cells), visited 32 at a time, one per lane; a ballot and a prefix count keep
-// the accepted ones in that order.  A cell whose candidates do not fit the
-// staging buffer reads them from global memory instead (same order).  The
-// distance test runs first and the exclusion test only for candidates inside
-// RLIST (the accepted set is the same); exclusions are compared as slots of
-// this list, and a virtual site is recognised by its label in the position's
-// w, so no candidate's global id is loaded.  The list is stored in the
-// nonbonded kernel's layout: T lanes per slot, slices of P = 32/T slots, entry
-// k of slot s (slice g) at (g*w_cap + k/T)*32 + (s%P)*T + k%T.  A slot that
-// needs more than w_cap rows records its need and raises the abort flag (the
-// host enlarges the storage and repeats the step).
 // The 13 neighbour cells of the half stencil in MAPS.f90:39-51 order.
 #define IBG_HALF_STENCIL                                                                                    \
   {{1, 0, 0}, {1, 1, 0},  {0, 1, 0},  {-1, 1, 0}, {1, 0, -1}, {1, 1, -1}, {0, 1, -1},                        \
@@ -683,19 +640,56 @@ __global__ void k_slot_of(__grid_constant__ const ListArgs L0, const ListArgs* c
 __constant__ int kStencil[13][3] = IBG_HALF_STENCIL;
 static const int kStencilHost[13][3] = IBG_HALF_STENCIL;  // the same, for host code
 
-// Candidates one block stages (positions and slots): 2,304 in FP32 (about 160
-// particles per cell), 1,152 in FP64, within 48 KB of static shared memory.
-// A staged slot carries its run (0..13) in bits 27..30, so lists hold fewer
-// than 2^27 particles.
+// NEW_NEIGHBOUR_WITHLIST.f90:34-123.  A unit of work is up to 32 particles of
+// one cell; a block takes units dynamically.  It stages the cell's candidates
+// in shared memory, in the reference's order: the cell's own slots, then the
+// slots of the 13 cells of the MAPS.f90:39-51 stencil, each run by decreasing
+// A (with more candidates than the stage holds, a stage at a time).
+//
+// Distances: a lane holds a particle and a warp walks 32 candidates at a time,
+// each one a broadcast from shared memory, leaving a bit per candidate and
+// lane for "inside RLIST" and for "outer group" (ListArgs::rgroupsq).  A unit
+// of 16 or 8 particles gives each two or four lanes, which take different
+// words of candidates, so that no lane is idle in a small group.
+//
+// Lists: bits of excluded partners are cleared (an exclusion's slot lies in one
+// of the runs, so its bit is known).  Every lane then writes the entries of its
+// own words one after another; counts of the words before them give their
+// places, so that they keep the candidates' order, the outer group's after the
+// others.
+//
+// The reference pairs a particle with the own-cell candidates below it only
+// (later in the staged order), and a virtual site with no other site.  The
+// list is stored in the nonbonded kernel's layout: T lanes per slot, slices of
+// P = 32/T slots, entry k of slot s (slice g) at (g*w_cap + k/T)*32 + (s%P)*T +
+// k%T.  A slot that needs more than w_cap rows records its need and raises the
+// abort flag (the host enlarges the storage and repeats the step).
+//
+// Minimum image: d - s with s the run's image shift (0 or +-L per axis).  For a
+// pair inside RLIST <= L/3 that shift is the nearest image, so s = ANINT(d/L)*L
+// exactly and d - s is the reference's d - ANINT(d/L)*L bit for bit; with any
+// other shift the distance is above RLIST either way.  A cell none of whose
+// runs wrapped has no shifts to subtract.
+//
+// Bound by instruction issue (160,000-bead melt: ~310 warp instructions a
+// particle for the distances, ~370 for writing the entries, the rest for
+// staging, exclusions and counts).  A warp per particle that tests 32
+// candidates at a time took ~1,400 (two ballots, prefix counts, exclusion
+// compares and the shift for every 32 tests): launch 276 us, now ~220; the
+// hybrid melt's two lists 405 us a rebuild with the cell sort, now 252.
+// Entries written by a lane per candidate, word by word, took 450 a particle;
+// by a lane per word, 1,150 (the words next to the particle are full).
+//
+// Candidates a block stages: 1,536 in FP32, 768 in FP64.  A staged slot carries
+// its run (0..13) in bits 27..30, so lists hold fewer than 2^27 particles.
 constexpr int kSlotMask = (1 << 27) - 1;
-// Entries of the outer group (ListArgs::rgroupsq) a list build holds back to
-// append after the others: per warp in the warp-per-particle build, per
-// thread in the thread-per-particle build.
-constexpr int kLateWarp = 48;
+// Entries of the outer group a thread of the thread-per-particle build holds
+// back to append after the others.
 constexpr int kLateThread = 24;
 template <typename R>
 struct ListStage {
-  static constexpr int cap = sizeof(R) == 4 ? 2304 : 1152;
+  static constexpr int words = sizeof(R) == 4 ? 48 : 24;  // of 32 candidates
+  static constexpr int cap = 32 * words;
 };
 
 template <typename R, int T, bool B>
@@ -704,43 +698,50 @@ __global__ void __launch_bounds__(256, 4) k_list_build_warp(__grid_constant__ co
   pdl_wait();
   pdl_trigger();
   using PT = typename Prec<R>::pos_t;
-  constexpr int kCap = ListStage<R>::cap;
-  constexpr int kWarps = 8;  // blockDim.x = 256
+  constexpr int kWords = ListStage<R>::words, kCap = ListStage<R>::cap;
+  constexpr int P = 32 / T;
   const Blk bk = blk<B>(bm);
   __shared__ ListArgs s_args;
   if (B) stage_args(&s_args, tab[bk.sys]);
   const ListArgs& L = B ? s_args : L0;
   Scalars* sc = L.sc;
   if (sc->skip || !(always || sc->rebuild)) return;
-  constexpr int P = 32 / T;
-  __shared__ PT s_pos[kCap];
-  __shared__ int s_slot[kCap];          // slot | run << 27
-  __shared__ int s_hi[14], s_pre[15];  // run u: slots s_hi[u] down, staged from s_pre[u]
-  __shared__ R s_sh[14][3];            // run u: periodic image shift, 0 or +-L per axis
-  __shared__ int s_exs[kWarps][20];    // each warp's particle's exclusions, as slots of this list
-  __shared__ int s_late[kWarps][kLateWarp];  // each warp's entries of the outer group (rgroupsq), in order
-  __shared__ int s_cell;
+  // candidates, 33 places per word: lanes that read different words at the
+  // same time then hit different banks
+  __shared__ PT s_pos[kWords * 33];
+  __shared__ int s_slot[kCap];
+  __shared__ unsigned s_in[kWords * 33], s_out[kWords * 33];  // [word][particle]: accepted, of them outer
+  __shared__ unsigned s_vs[kWords];      // virtual sites among a word's candidates
+  __shared__ int s_hi[14], s_pre[15];    // run u: slots s_hi[u] down, candidates from s_pre[u]
+  __shared__ R s_sh[14][3];              // run u: periodic image shift
+  __shared__ int s_ex[32][20], s_ne[32], s_cnt[32], s_i[32];
+  __shared__ int s_n[256];               // [share of the words][particle]: entries, the outer group's << 16
+  __shared__ int s_unit[2], s_wrap;
   const int nx = sc->ncell[L.which][0], ny = sc->ncell[L.which][1], nz = sc->ncell[L.which][2];
+  // units per cell: one where there are cells enough for two per block (its
+  // groups of particles then share one stage), else one per group
   const int ncells = nx * ny * nz;
+  const int G = ncells >= 2 * bk.g ? 1 : max(1, (sc->cell_max[L.which] + 31) / 32);
+  const int nunits = ncells * G;
   R b[3], bi[3], b2[3];
   box_of<R>(sc, b, bi, b2);
   const R rlsq = sizeof(R) == 4 ? (R)L.rlistsq : (R)L.rlistsqd;
   const R rg = L.rgroupsq > 0.f ? (R)L.rgroupsq : rlsq;
   const PT* pos = (const PT*)L.pos4;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const unsigned below = (1u << lane) - 1u;
-  int* late = s_late[warp];
+  constexpr int kWarps = 8;  // blockDim.x = 256
   const int cap = L.w_cap * T;  // entries a slot may hold
-  int* exs = s_exs[warp];
   int most = 0;  // most rows of any particle this lane closed
-  for (;;) {
-    __syncthreads();  // the previous cell's staging is no longer read
-    if (threadIdx.x == 0) s_cell = (int)atomicAdd(&sc->work[2 + L.which], 1u);
-    __syncthreads();
-    const int c0 = s_cell;
-    if (c0 >= ncells) break;
+  if (threadIdx.x == 0) s_unit[0] = (int)atomicAdd(&sc->work[2 + L.which], 1u);
+  for (int turn = 0;; turn ^= 1) {
+    __syncthreads();  // the unit's number is there; the last one's stage is no longer read
+    const int unit = s_unit[turn];
+    if (unit >= nunits) break;
+    if (threadIdx.x == 0) s_unit[turn ^ 1] = (int)atomicAdd(&sc->work[2 + L.which], 1u);  // the next one's, meanwhile
+    const int c0 = G == 1 ? unit : unit / G;
     const int first = L.cell_start[c0], last = L.cell_start[c0 + 1];
-    if (first == last) continue;
+    const int start = first + (unit - c0 * G) * 32;
+    if (start >= last) continue;
     if (warp == 0) {
       // run 0: the own cell from its last slot down; runs 1..13: the stencil
       // cells, each from its last slot down; exclusive prefix of the lengths
@@ -769,6 +770,7 @@ __global__ void __launch_bounds__(256, 4) k_list_build_warp(__grid_constant__ co
         const int y = __shfl_up_sync(0xffffffffu, incl, o);
         if (lane >= o) incl += y;
       }
+      const unsigned wraps = __ballot_sync(0xffffffffu, (w[0] | w[1] | w[2]) != 0);
       if (lane < 14) {
         s_hi[lane] = hi;
         s_pre[lane] = incl - len;
@@ -776,115 +778,183 @@ __global__ void __launch_bounds__(256, 4) k_list_build_warp(__grid_constant__ co
         for (int q = 0; q < 3; ++q) s_sh[lane][q] = w[q] > 0 ? b[q] : (w[q] < 0 ? -b[q] : (R)0);
       }
       if (lane == 13) s_pre[14] = incl;
+      if (lane == 0) s_wrap = wraps != 0;
     }
-    __syncthreads();
-    const int total = s_pre[14];
-    // staged index v -> slot | run << 27, the run being the largest u with
-    // s_pre[u] <= v (that run is not empty)
-    auto slot_at = [&](int v) {
-      int lo = 0, hi = 13;
-      while (lo < hi) {
-        const int mid = (lo + hi + 1) >> 1;
-        if (s_pre[mid] <= v) lo = mid;
-        else hi = mid - 1;
+    bool staged = false;
+    for (int s0 = start; s0 < last; s0 += 32 * G) {
+      const int np = min(32, last - s0);
+      if (s0 > start) __syncthreads();  // the group before is done
+      if (warp == 1) {
+        int i = 0, ne = 0;
+        if (lane < np) {
+          i = L.idx[L.sorted[s0 + lane]];
+          ne = min(L.excl_n[i], 20);
+        }
+        s_i[lane] = i;
+        s_ne[lane] = ne;
+        s_cnt[lane] = 0;
       }
-      return (s_hi[lo] - (v - s_pre[lo])) | (lo << 27);
-    };
-    const bool staged = total <= kCap;
-    if (staged) {
-      for (int v = threadIdx.x; v < total; v += blockDim.x) {
-        const int tu = slot_at(v);
-        s_slot[v] = tu;
-        s_pos[v] = pos[tu & kSlotMask];
+      __syncthreads();
+      const int total = s_pre[14];
+      const bool wrap = s_wrap != 0;
+      // the particles' exclusions, as slots of this list
+      for (int k = threadIdx.x; k < 32 * 20; k += blockDim.x) {
+        const int p = k / 20, e = k - 20 * p;
+        if (e >= s_ne[p]) continue;
+        const int gs = L.gslot[L.excl[(size_t)s_i[p] * 20 + e]];
+        s_ex[p][e] = (gs & 1) == L.which ? gs >> 1 : -1;
       }
-    }
-    __syncthreads();
-    for (int s = first + warp; s < last; s += kWarps) {
-      const int g = s / P;
-      const long long base = (long long)g * L.w_cap * 32 + (s % P) * T;
-      const int a = L.sorted[s];
-      const int i = L.idx[a];
-      const PT pi = staged ? s_pos[last - 1 - s] : pos[s];
-      const int ne = L.excl_n[i];
-      if (lane < ne) {
-        const int gs = L.gslot[L.excl[(size_t)i * 20 + lane]];
-        exs[lane] = (gs & 1) == L.which ? gs >> 1 : -1;
-      }
-      __syncwarp();
-      // the first four exclusions in registers (a bead of a chain has four
-      // 1-2 and 1-3 partners), the rest from shared memory
-      const int e0 = ne > 0 ? exs[0] : -1, e1 = ne > 1 ? exs[1] : -1, e2 = ne > 2 ? exs[2] : -1,
-                e3 = ne > 3 ? exs[3] : -1;
-      const bool i_vs = L.hybrid && i >= L.natoms;
-      int cnt = 0, nlate = 0;
-      // minimum image: d - s with s the run's image shift.  For a pair inside
-      // RLIST <= L/3 that shift is the nearest image, so s = ANINT(d/L)*L
-      // exactly and d - s is the reference's d - ANINT(d/L)*L bit for bit;
-      // with any other shift the distance is above RLIST either way.
-      for (int v0 = last - s; v0 < total; v0 += 32) {
-        const int v = v0 + lane;
-        bool ok = false;
-        int t = -1;
-        R r2 = (R)0;
-        if (v < total) {
-          PT pj;
-          int tu;
-          if (staged) {
-            tu = s_slot[v];
-            pj = s_pos[v];
-          } else {
-            tu = slot_at(v);
-            pj = pos[tu & kSlotMask];
+      // this lane's particle in the distance pass, and its share of the words
+      const int PL = np > 16 ? 32 : (np > 8 ? 16 : 8), SL = 32 / PL;
+      const int p1 = lane & (PL - 1), sub = lane / PL;
+      const int own = last - 1 - (s0 + p1);  // its place among the candidates: it pairs with later ones
+      PT pi;
+      if (p1 < np) pi = pos[s0 + p1];
+      else { pi.x = pi.y = pi.z = 0; pi.w = Prec<R>::tbits(0); }
+      const unsigned site = L.hybrid && p1 < np && s_i[p1] >= L.natoms ? 0xffffffffu : 0u;
+      for (int base = 0; base < total; base += kCap) {
+        const int nv = min(kCap, total - base), W = (nv + 31) / 32;
+        if (base > 0) __syncthreads();  // the stage before is no longer read
+        for (int w = staged ? W : warp; w < W; w += kWarps) {
+          const int v = 32 * w + lane;
+          PT q;
+          bool vs = false;
+          if (v < nv) {
+            // the run of candidate base + v: the largest u with s_pre[u] <= it
+            // (that run is not empty)
+            int lo = 0;
+  #pragma unroll
+            for (int step = 8; step > 0; step >>= 1)
+              if (lo + step < 14 && s_pre[lo + step] <= base + v) lo += step;
+            const int t = s_hi[lo] - (base + v - s_pre[lo]);
+            s_slot[v] = t;
+            q = pos[t];
+            vs = (Prec<R>::bits(q.w) >> 16) == 3;
+            q.w = Prec<R>::tbits(lo);
+          } else {  // beyond the candidates: farther than any RLIST
+            q.x = q.y = q.z = (R)1e18;
+            q.w = Prec<R>::tbits(0);
           }
-          t = tu & kSlotMask;
-          const R* sh = s_sh[tu >> 27];
-          R d0 = pi.x - pj.x, d1 = pi.y - pj.y, d2 = pi.z - pj.z;
-          d0 = d0 - sh[0];
-          d1 = d1 - sh[1];
-          d2 = d2 - sh[2];
-          r2 = d0 * d0;
-          r2 = r2 + d1 * d1;
-          r2 = r2 + d2 * d2;
-          ok = r2 < rlsq && !(i_vs && (Prec<R>::bits(pj.w) >> 16) == 3) && t != e0 && t != e1 && t != e2 &&
-               t != e3;
-          if (ok && ne > 4)
-            for (int e = 4; e < ne; ++e) ok &= exs[e] != t;
+          s_pos[33 * w + lane] = q;
+          const unsigned m = __ballot_sync(0xffffffffu, vs);
+          if (lane == 0) s_vs[w] = m;
         }
-        // entries of the outer group go to the warp's stage while it has
-        // room (the rest are written in place, which only mixes the groups)
-        const bool outer = ok && r2 >= rg;
-        const unsigned mo = __ballot_sync(0xffffffffu, outer);
-        const int po = __popc(mo & below), room = kLateWarp - nlate;
-        const bool staged_late = outer && po < room;
-        const bool now = ok && !staged_late;
-        const unsigned m = __ballot_sync(0xffffffffu, now);
-        if (now) {
-          const int k = cnt + __popc(m & below);
-          if (k < cap) ((int*)L.entries)[base + (long long)(k / T) * 32 + (k % T)] = t;
+        staged = total <= kCap;
+        __syncthreads();
+        // the words from w1 on are this lane's, nw of them: consecutive ones, so
+        // that its entries are consecutive in its particle's list
+        const int nw = (W + kWarps * SL - 1) / (kWarps * SL), share = warp * SL + sub, w1 = share * nw;
+        for (int q0 = 0; q0 < nw; ++q0) {
+          const int w = w1 + q0;
+          if (!__any_sync(0xffffffffu, w < W)) break;
+          const PT* cand = s_pos + 33 * min(w, W - 1);
+          unsigned m = 0, far = 0;
+          auto test = [&](R d0, R d1, R d2, unsigned bit) {
+            R r2 = d0 * d0;
+            r2 = r2 + d1 * d1;
+            r2 = r2 + d2 * d2;
+            if (r2 < rlsq) m |= bit;
+            if (r2 >= rg) far |= bit;
+          };
+          if (!wrap) {
+  #pragma unroll 16
+            for (int k = 0; k < 32; ++k) {
+              const PT q = cand[k];
+              test(pi.x - q.x, pi.y - q.y, pi.z - q.z, 1u << k);
+            }
+          } else {
+  #pragma unroll 8
+            for (int k = 0; k < 32; ++k) {
+              const PT q = cand[k];
+              const R* sh = s_sh[Prec<R>::bits(q.w)];
+              R d0 = pi.x - q.x, d1 = pi.y - q.y, d2 = pi.z - q.z;
+              d0 = d0 - sh[0];
+              d1 = d1 - sh[1];
+              d2 = d2 - sh[2];
+              test(d0, d1, d2, 1u << k);
+            }
+          }
+          if (w < W && p1 < np) {
+            const int skip = own + 1 - (base + 32 * w);  // candidates of this word up to the particle itself
+            if (skip > 0) m = skip >= 32 ? 0u : m & ~((1u << skip) - 1u);
+            m &= ~(site & s_vs[w]);
+            s_in[33 * w + p1] = m;
+            s_out[33 * w + p1] = m & far;
+          }
         }
-        if (staged_late) late[nlate + po] = t;
-        cnt += __popc(m);
-        nlate += min(__popc(mo), room);
-      }
-      __syncwarp();
-      for (int q = lane; q < nlate; q += 32) {
-        const int k = cnt + q;
-        if (k < cap) ((int*)L.entries)[base + (long long)(k / T) * 32 + (k % T)] = late[q];
-      }
-      cnt += nlate;
-      if (lane == 0) {
-        L.counts[s] = cnt;
-        if (cnt >= L.maxnab) atomicOr(&sc->err, EB_LIST_OVERFLOW);
-        const int rows = (cnt + T - 1) / T;
-        most = max(most, rows);
-        atomicMax(&L.slice_w[g], rows);
-        if (rows > L.w_cap) {
-          atomicMax(&sc->need_rows[L.which], rows);
-          sc->abort = 1;
-          sc->skip = 1;
+        __syncthreads();
+        // an excluded slot lies in one of the runs: clear its candidate's bit
+        // (warp: which exclusion; lane: whose)
+        const bool closing = base + kCap >= total;
+        for (int e = warp; e < 20; e += kWarps) {
+          const int t = e < s_ne[lane] ? s_ex[lane][e] : -1;
+          if (!__any_sync(0xffffffffu, t >= 0)) continue;
+          for (int u = 0; u < 14; ++u) {
+            const int hi = s_hi[u], pre = s_pre[u], v = pre + hi - t - base;
+            if (t < 0 || t > hi || hi - t >= s_pre[u + 1] - pre || v < 0 || v >= nv) continue;
+            atomicAnd(&s_in[33 * (v >> 5) + lane], ~(1u << (v & 31)));
+            atomicAnd(&s_out[33 * (v >> 5) + lane], ~(1u << (v & 31)));
+          }
+        }
+        __syncthreads();
+        // how many entries each lane's words hold, the outer group's in the upper
+        // half, and how many come before them
+        const int last_w = min(W, w1 + nw);
+        int mine = 0;
+        if (p1 < np)
+          for (int w = w1; w < last_w; ++w) {
+            const unsigned m = s_in[33 * w + p1], o = closing ? s_out[33 * w + p1] : 0u;
+            mine += __popc(m & ~o) + (__popc(o) << 16);
+          }
+        s_n[share * PL + p1] = mine;
+        __syncthreads();
+        int before = 0, all = 0;
+        for (int r = 0; r < kWarps * SL; ++r) {
+          const int x = s_n[r * PL + p1];
+          if (r < share) before += x;
+          all += x;
+        }
+        if (p1 < np) {
+          const int s = s0 + p1, g = s / P, cnt0 = s_cnt[p1];
+          int* row = L.entries + (long long)g * L.w_cap * 32 + (s % P) * T;
+          int ki = cnt0 + (before & 0xffff), ko = cnt0 + (all & 0xffff) + (before >> 16);
+          // the lane's bits one after another, whatever word they are in (a list
+          // that another stage of candidates follows is stored as found, which
+          // only mixes the groups)
+          int w = w1 - 1;
+          unsigned m = 0, o = 0;
+          for (int left = (mine & 0xffff) + (mine >> 16); left > 0;) {
+            if (m == 0) {
+              ++w;
+              m = s_in[33 * w + p1];
+              o = closing ? s_out[33 * w + p1] : 0u;
+              continue;
+            }
+            const int bit = __ffs(m) - 1;
+            m &= m - 1u;
+            --left;
+            const int k = (o >> bit) & 1u ? ko++ : ki++;
+            if (k < cap) row[(k / T) * 32 + (k % T)] = s_slot[32 * w + bit];
+          }
+          if (share == 0 && closing) {
+            const int cnt = cnt0 + (all & 0xffff) + (all >> 16);
+            L.counts[s] = cnt;
+            if (cnt >= L.maxnab) atomicOr(&sc->err, EB_LIST_OVERFLOW);
+            const int rows = (cnt + T - 1) / T;
+            most = max(most, rows);
+            atomicMax(&L.slice_w[g], rows);
+            if (rows > L.w_cap) {
+              atomicMax(&sc->need_rows[L.which], rows);
+              sc->abort = 1;
+              sc->skip = 1;
+            }
+          }
+        }
+        if (!closing) {
+          __syncthreads();  // every lane has read the counts
+          if (share == 0 && p1 < np) s_cnt[p1] += (all & 0xffff) + (all >> 16);
         }
       }
-      __syncwarp();  // exs is rewritten for the next particle
     }
   }
   if (most > 0) atomicMax(&sc->rows_max[L.which], most);
@@ -2142,45 +2212,42 @@ __device__ bool inside_as_fp64(const NBArgs<float>& A, const Scalars* sc, int gi
 
 // A pair the FP32 kernel left at the cutoff: decided as the FP64 path decides
 // it (inside_as_fp64) and, when inside, computed with the FP32 kernel's pair
-// arithmetic.  f: i's share of the force in fixed point, e: V_NB(1..3) and the
-// six virial terms.  False when the pair does not count.
-__device__ __noinline__ bool near_pair(const NBArgs<float>& A, const int4& nk, float ux, float uy, float uz, long long (&f)[3],
-                          long long (&e)[9], unsigned& err) {
+// arithmetic.  force(c, q): i's share of component c in fixed point; term(k,
+// q): V_NB(1..3) and the six virial terms, k = 0..8.
+template <typename Force, typename Term>
+__device__ __forceinline__ void near_pair(const NBArgs<float>& A, const int4& nk, float ux, float uy, float uz,
+                                          unsigned& err, Force&& force, Term&& term) {
   const int4 pi = A.posq[nk.x], pj = A.posq[nk.y];
   const float d0 = (float)(int)((unsigned)pi.x - (unsigned)pj.x) * ux;
   const float d1 = (float)(int)((unsigned)pi.y - (unsigned)pj.y) * uy;
   const float d2 = (float)(int)((unsigned)pi.z - (unsigned)pj.z) * uz;
   const float r2 = __fmaf_rn(d2, d2, __fmaf_rn(d1, d1, d0 * d0));
-  if (!inside_as_fp64(A, A.sc, nk.z, nk.w, r2)) return false;
+  if (!inside_as_fp64(A, A.sc, nk.z, nk.w, r2)) return;
   const int ti = pi.w & 0xffff, li = pi.w >> 16, tj = pj.w & 0xffff, lj = pj.w >> 16;
   const int4 pt = A.ptab[ti * A.ntype + tj];
-  if (!pt.w) { err |= EB_MISSING_TABLE; return false; }
+  if (!pt.w) { err |= EB_MISSING_TABLE; return; }
   const float r = r2 * rsqrtf(r2);
   const float ib = __int_as_float(pt.z);
   const int ni = (int)(r * ib);
-  if (ni > pt.y) { err |= EB_TABLE_RANGE; return false; }
+  if (ni > pt.y) { err |= EB_TABLE_RANGE; return; }
   const int row = pt.x + ni;
   const float alpha = (r - A.tx[row]) * ib;
   const float2 a0 = ((const float2*)A.tfp)[row], a1 = ((const float2*)A.tfp)[row + 1];
   const float fij = __fmaf_rn(a1.x - a0.x, alpha, a0.x);
   const float vij = __fmaf_rn(a1.y - a0.y, alpha, a0.y);
-  if (!(fabsf(fij) * r < 0.99f * kFixMax)) { err |= EB_FIXED; return false; }
+  if (!(fabsf(fij) * r < 0.99f * kFixMax)) { err |= EB_FIXED; return; }
   const float fx = fij * d0, fy = fij * d1, fz = fij * d2;
-  f[0] = __float2ll_rn(fx * kFixScale);
-  f[1] = __float2ll_rn(fy * kFixScale);
-  f[2] = __float2ll_rn(fz * kFixScale);
-  const bool lab3 = li == 3 || lj == 3;
-  const long long qe = fixq<24>(vij, err);
-  e[0] = li == 1 ? qe : 0;
-  e[1] = li == 2 && lj == 2 ? qe : 0;
-  e[2] = li != 1 && lab3 ? qe : 0;
-  e[3] = fixq<24>(fx * d0, err);
-  e[4] = fixq<24>(fy * d1, err);
-  e[5] = fixq<24>(fz * d2, err);
-  e[6] = fixq<24>(fy * d0, err);
-  e[7] = fixq<24>(fz * d0, err);
-  e[8] = fixq<24>(fz * d1, err);
-  return true;
+  force(0, __float2ll_rn(fx * kFixScale));
+  force(1, __float2ll_rn(fy * kFixScale));
+  force(2, __float2ll_rn(fz * kFixScale));
+  // V_NB(1) for an atom i, V_NB(2) for two beads, V_NB(3) with a site
+  if (li == 1 || li == 3 || lj == 3 || lj == 2) term(li == 1 ? 0 : (li == 3 || lj == 3 ? 2 : 1), fixq<24>(vij, err));
+  term(3, fixq<24>(fx * d0, err));
+  term(4, fixq<24>(fy * d1, err));
+  term(5, fixq<24>(fz * d2, err));
+  term(6, fixq<24>(fy * d0, err));
+  term(7, fixq<24>(fz * d0, err));
+  term(8, fixq<24>(fz * d1, err));
 }
 
 // More pairs came at the cutoff than their buffer holds: record the need and
@@ -2206,34 +2273,33 @@ __global__ void __launch_bounds__(256) k_nb_near(__grid_constant__ const NBArgs<
   const NBArgs<float>& A = B ? *tab[bk.sys] : A0;
   Scalars* sc = A.sc;
   if (A.near_in_collect || nb_idle(A)) return;
-  __shared__ long long red[9 + 9 * 8];
   const unsigned n = sc->near_n[A.work];
   if (n > (unsigned)A.near_cap) {
     __syncthreads();  // every thread has read the count
     if (threadIdx.x == 0) near_overflow(sc, A.work, n);
     return;
   }
+  __shared__ unsigned long long s_sum[9];
+  if (threadIdx.x < 9) s_sum[threadIdx.x] = 0ull;
+  __syncthreads();
   const float ux = (float)(sc->box[0] * 0x1p-32), uy = (float)(sc->box[1] * 0x1p-32), uz = (float)(sc->box[2] * 0x1p-32);
   unsigned err = 0;
-  long long acc[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
   for (unsigned k = threadIdx.x; k < n; k += blockDim.x) {
     const int4 nk = A.near[k];
-    long long f[3], e[9];
-    if (!near_pair(A, nk, ux, uy, uz, f, e, err)) continue;
     unsigned long long* fsi = (unsigned long long*)A.fsort + fs_at(nk.x);
     unsigned long long* fsj = (unsigned long long*)A.fsort + fs_at(nk.y);
-#pragma unroll
-    for (int c = 0; c < 3; ++c) {
-      atomicAdd(fsi + 32 * c, (unsigned long long)f[c]);
-      atomicAdd(fsj + 32 * c, (unsigned long long)(-f[c]));
-    }
-#pragma unroll
-    for (int c = 0; c < 9; ++c) acc[c] += e[c];
+    near_pair(
+        A, nk, ux, uy, uz, err,
+        [&](int c, long long f) {
+          atomicAdd(fsi + 32 * c, (unsigned long long)f);
+          atomicAdd(fsj + 32 * c, (unsigned long long)(-f));
+        },
+        [&](int t, long long e) { atomicAdd(&s_sum[t], (unsigned long long)e); });
   }
   if (err) atomicOr(&sc->err, err);
-  block_sums<9>(acc, red);
-  if (threadIdx.x < 9 && red[threadIdx.x] != 0)
-    atomicAdd(&sc->nbacc[A.work][threadIdx.x], (unsigned long long)red[threadIdx.x]);
+  __syncthreads();
+  if (threadIdx.x < 9 && s_sum[threadIdx.x] != 0)
+    atomicAdd(&sc->nbacc[A.work][threadIdx.x], s_sum[threadIdx.x]);
   __syncthreads();
   if (threadIdx.x == 0) sc->near_n[A.work] = 0u;
 }
@@ -2260,7 +2326,7 @@ struct CollectArgs {
 };
 
 template <typename R, bool B>
-__global__ void __launch_bounds__(256, 5) k_nb_collect(__grid_constant__ const CollectArgs<R> C0, const CollectArgs<R>* const* tab,
+__global__ void __launch_bounds__(256, 4) k_nb_collect(__grid_constant__ const CollectArgs<R> C0, const CollectArgs<R>* const* tab,
                              const BlockMap bm) {
   using P = Prec<R>;
   pdl_wait();
@@ -2294,18 +2360,16 @@ __global__ void __launch_bounds__(256, 5) k_nb_collect(__grid_constant__ const C
         const int4 nk = A.near[k];
         const bool own_i = (nk.x >> 8) == bk.b, own_j = (nk.y >> 8) == bk.b;
         if (!own_i && !own_j) continue;
-        long long f[3], e[9];
         unsigned err = 0;
-        if (near_pair(A, nk, ux, uy, uz, f, e, err)) {
-#pragma unroll
-          for (int c = 0; c < 3; ++c) {
-            if (own_i) atomicAdd(&s_near[c][nk.x & 255], (unsigned long long)f[c]);
-            if (own_j) atomicAdd(&s_near[c][nk.y & 255], (unsigned long long)(-f[c]));
-          }
-          if (own_i)
-            for (int c = 0; c < 9; ++c)
-              if (e[c] != 0) atomicAdd(&sc->nbacc[C.work][c], (unsigned long long)e[c]);
-        }
+        near_pair(
+            A, nk, ux, uy, uz, err,
+            [&](int c, long long f) {
+              if (own_i) atomicAdd(&s_near[c][nk.x & 255], (unsigned long long)f);
+              if (own_j) atomicAdd(&s_near[c][nk.y & 255], (unsigned long long)(-f));
+            },
+            [&](int t, long long e) {
+              if (own_i && e != 0) atomicAdd(&sc->nbacc[C.work][t], (unsigned long long)e);
+            });
         if (own_i && err) atomicOr(&sc->err, err);
       }
       __syncthreads();
