@@ -2494,12 +2494,28 @@ __device__ __forceinline__ void addf(typename Prec<A>::acc_t* F, int i, const do
   P::add(&F[3 * (size_t)i + 2], P::from_double(f[2], err));
 }
 
+// Two shares of one particle's force, sa * a + sb * b (signs +-1), each rounded
+// to the accumulator on its own and added in one update per component.
+template <typename A>
+__device__ __forceinline__ void addf2(typename Prec<A>::acc_t* F, int i, const double* a, const double* b, double sa,
+                                      double sb, unsigned* err) {
+  using P = Prec<A>;
+#pragma unroll
+  for (int c = 0; c < 3; ++c)
+    P::add(&F[3 * (size_t)i + c], P::from_double(sa * a[c], err) + P::from_double(sb * b[c], err));
+}
+
 // BONDS.inc:3-57, ANGLES.inc:2-75, TORSIONS.inc:1-152, OUTOFPLANES.inc:1-141
 // with one thread per term; the four term kinds share the grid.  The bonded
 // geometry is evaluated in FP64 on both paths: acos near straight angles and
 // trans dihedrals amplifies REAL*4 rounding (about 1e-5 of the largest force
 // in a strained chain), while the terms are few; the forces are summed in the
-// path's accumulator (64-bit fixed point on the FP32 path).
+// path's accumulator (64-bit fixed point on the FP32 path).  Lengths and sines
+// that only scale a force are divided by through one reciprocal each (an angle
+// had 20 FP64 divisions, a torsion 27, of ~20 instructions; now 6 and 14); the
+// cosines of angles and dihedrals keep the reference's divisions, which their
+// arc cosine would amplify near straight and planar ones.  A particle's two
+// shares of a term are added in one update.
 template <typename A, bool BA>
 __global__ void __launch_bounds__(256) k_bonded(__grid_constant__ const BondedArgs<A> B0, const BondedArgs<A>* const* tab,
                                                 const BlockMap bm) {
@@ -2527,12 +2543,12 @@ __global__ void __launch_bounds__(256) k_bonded(__grid_constant__ const BondedAr
       const R rij = r_sqrt(rsq);
       const int t = e.z;
       const float4* T = B.tb + B.tb_off[t];
-      const R bin = (R)B.tb_bin[t];
-      int k = fint((rij - (R)T[0].x) / bin);
+      const R ibin = (R)1 / (R)B.tb_bin[t];
+      int k = fint((rij - (R)T[0].x) * ibin);
       if (k > B.tb_ndat[t]) { ++overext; k = B.tb_ndat[t]; }
       else if (k < 0) k = 0;
       const float4 r0 = T[k], r1 = T[k + 1];
-      const R alpha = (rij - (R)r0.x) / bin;
+      const R alpha = (rij - (R)r0.x) * ibin;
       const R fij = lerp_mixed<R>((R)r0.y, (R)r1.y, alpha);
       const R vij = lerp_mixed<R>((R)r0.z, (R)r1.z, alpha);
       acc[e.w - 1] += (double)vij;
@@ -2548,6 +2564,7 @@ __global__ void __launch_bounds__(256) k_bonded(__grid_constant__ const BondedAr
       for (int c = 0; c < 3; ++c) { ij[c] = ri[c] - rj[c]; kj[c] = rk[c] - rj[c]; }
       const R rij = r_sqrt((ij[0] * ij[0] + ij[1] * ij[1]) + ij[2] * ij[2]);
       const R rkj = r_sqrt((kj[0] * kj[0] + kj[1] * kj[1]) + kj[2] * kj[2]);
+      const R iij = (R)1 / rij, ikj = (R)1 / rkj;
       R ct = ((ij[0] * kj[0] + ij[1] * kj[1]) + ij[2] * kj[2]) / rij / rkj;
       ct = ct > (R)1 ? (R)1 : (ct < (R)-1 ? (R)-1 : ct);  // rounding of a straight angle (the oracle clamps too)
       const R theta = r_acos(ct) * (R)B.r2d;
@@ -2556,14 +2573,15 @@ __global__ void __launch_bounds__(256) k_bonded(__grid_constant__ const BondedAr
       m[1] = -(-ij[0] * kj[2] + ij[2] * kj[0]);
       m[2] = -(ij[0] * kj[1] - ij[1] * kj[0]);
       const R rm = r_sqrt((m[0] * m[0] + m[1] * m[1]) + m[2] * m[2]);
-      for (int c = 0; c < 3; ++c) m[c] = m[c] / rm;
+      const R irm = (R)1 / rm;
+      for (int c = 0; c < 3; ++c) m[c] = m[c] * irm;
       R nn[3], ss[3];
-      nn[0] = (m[1] * ij[2] - m[2] * ij[1]) / rij;
-      nn[1] = (-m[0] * ij[2] + m[2] * ij[0]) / rij;
-      nn[2] = (m[0] * ij[1] - m[1] * ij[0]) / rij;
-      ss[0] = -(m[1] * kj[2] - m[2] * kj[1]) / rkj;
-      ss[1] = -(-m[0] * kj[2] + m[2] * kj[0]) / rkj;
-      ss[2] = -(m[0] * kj[1] - m[1] * kj[0]) / rkj;
+      nn[0] = (m[1] * ij[2] - m[2] * ij[1]) * iij;
+      nn[1] = (-m[0] * ij[2] + m[2] * ij[0]) * iij;
+      nn[2] = (m[0] * ij[1] - m[1] * ij[0]) * iij;
+      ss[0] = -(m[1] * kj[2] - m[2] * kj[1]) * ikj;
+      ss[1] = -(-m[0] * kj[2] + m[2] * kj[0]) * ikj;
+      ss[2] = -(m[0] * kj[1] - m[1] * kj[0]) * ikj;
       const float4* T = B.ta + B.ta_off[t];
       const R bin = (R)B.ta_bin[t];
       int k = fint(theta / bin);
@@ -2581,14 +2599,13 @@ __global__ void __launch_bounds__(256) k_bonded(__grid_constant__ const BondedAr
       acc[3 + lab - 1] += (double)vijk;
       R fI[3], fK[3], mI[3], mK[3];
       for (int c = 0; c < 3; ++c) {
-        fI[c] = fijk * nn[c] / rij;
-        fK[c] = fijk * ss[c] / rkj;
+        fI[c] = fijk * nn[c] * iij;
+        fK[c] = fijk * ss[c] * ikj;
         mI[c] = -fI[c]; mK[c] = -fK[c];
       }
       addf<A>(B.fb, e.x, fI, err);
       addf<A>(B.fb, e.z, fK, err);
-      addf<A>(B.fb, e.y, mK, err);
-      addf<A>(B.fb, e.y, mI, err);
+      addf2<A>(B.fb, e.y, mK, mI, (R)1, (R)1, err);
     } else if (u < B.nb + B.na + B.nt) {  // -------- torsion
       const int q = u - B.nb - B.na;
       const int4 e = B.tors[q];
@@ -2599,7 +2616,8 @@ __global__ void __launch_bounds__(256) k_bonded(__grid_constant__ const BondedAr
       R rij = r_sqrt((ij[0] * ij[0] + ij[1] * ij[1]) + ij[2] * ij[2]);
       const R rjk = r_sqrt((jk[0] * jk[0] + jk[1] * jk[1]) + jk[2] * jk[2]);
       R rkl = r_sqrt((kl[0] * kl[0] + kl[1] * kl[1]) + kl[2] * kl[2]);
-      R m[3], nn[3], cosm = 0, sinm = 0, cotanm = 0, cosn = 0, sinn = 0, cotann = 0;
+      const R ijk = (R)1 / rjk;
+      R m[3], nn[3], cosm = 0, isinm = 0, cotanm = 0, cosn = 0, isinn = 0, cotann = 0, iij = 0, ikl = 0;
       auto crossm = [&]() {
         m[0] = ij[1] * jk[2] - ij[2] * jk[1];
         m[1] = -ij[0] * jk[2] + ij[2] * jk[0];
@@ -2620,9 +2638,10 @@ __global__ void __launch_bounds__(256) k_bonded(__grid_constant__ const BondedAr
       }
       if (rm > (R)0 || rm == (R)0) {
         for (int c = 0; c < 3; ++c) m[c] = m[c] / rm;
-        cosm = ((ij[0] * jk[0] + ij[1] * jk[1]) + ij[2] * jk[2]) / rij / rjk;
-        sinm = r_sqrt((R)1 - cosm * cosm);
-        cotanm = cosm / sinm;
+        iij = (R)1 / rij;
+        cosm = ((ij[0] * jk[0] + ij[1] * jk[1]) + ij[2] * jk[2]) * iij * ijk;
+        isinm = (R)1 / r_sqrt((R)1 - cosm * cosm);
+        cotanm = cosm * isinm;
       }
       crossn();
       R rn = r_sqrt((nn[0] * nn[0] + nn[1] * nn[1]) + nn[2] * nn[2]);
@@ -2634,9 +2653,10 @@ __global__ void __launch_bounds__(256) k_bonded(__grid_constant__ const BondedAr
       }
       if (rn > (R)0 || rn == (R)0) {
         for (int c = 0; c < 3; ++c) nn[c] = nn[c] / rn;
-        cosn = ((jk[0] * kl[0] + jk[1] * kl[1]) + jk[2] * kl[2]) / rjk / rkl;
-        sinn = r_sqrt((R)1 - cosn * cosn);
-        cotann = cosn / sinn;
+        ikl = (R)1 / rkl;
+        cosn = ((jk[0] * kl[0] + jk[1] * kl[1]) + jk[2] * kl[2]) * ijk * ikl;
+        isinn = (R)1 / r_sqrt((R)1 - cosn * cosn);
+        cotann = cosn * isinn;
       }
       R cost = (m[0] * nn[0] + m[1] * nn[1]) + m[2] * nn[2];
       const R signt = -((m[0] * kl[0] + m[1] * kl[1]) + m[2] * kl[2]);
@@ -2660,21 +2680,16 @@ __global__ void __launch_bounds__(256) k_bonded(__grid_constant__ const BondedAr
         vijkl = (R)r0.z * ((R)1.0 - alpha) + alpha * (R)r1.z;
       }
       acc[6 + tl.y - 1] += (double)vijkl;
-      R f1[3], f4[3], f12[3], a[3];
+      R f1[3], f4[3], f12[3];
       for (int c = 0; c < 3; ++c) {
-        f1[c] = -(fijkl * m[c] / sinm / rij);
-        f4[c] = fijkl * nn[c] / sinn / rkl;
-        f12[c] = fijkl * (cotanm * m[c] + cotann * nn[c]) / rjk;
+        f1[c] = -(fijkl * m[c] * isinm * iij);
+        f4[c] = fijkl * nn[c] * isinn * ikl;
+        f12[c] = fijkl * (cotanm * m[c] + cotann * nn[c]) * ijk;
       }
       addf<A>(B.fb, e.x, f1, err);
       addf<A>(B.fb, e.w, f4, err);
-      for (int c = 0; c < 3; ++c) a[c] = -f1[c];
-      addf<A>(B.fb, e.y, a, err);
-      addf<A>(B.fb, e.y, f12, err);
-      for (int c = 0; c < 3; ++c) a[c] = -f4[c];
-      addf<A>(B.fb, e.z, a, err);
-      for (int c = 0; c < 3; ++c) a[c] = -f12[c];
-      addf<A>(B.fb, e.z, a, err);
+      addf2<A>(B.fb, e.y, f1, f12, (R)-1, (R)1, err);
+      addf2<A>(B.fb, e.z, f4, f12, (R)-1, (R)-1, err);
     } else {  // ------------------------------------------ out of plane
       const int q = u - B.nb - B.na - B.nt;
       const int4 e = B.oops[q];
