@@ -130,7 +130,6 @@ struct DevList {
   int near_cap = 0;
   size_t pos_bytes = 0;
   // tables of this list
-  int *ltab = nullptr, *toff = nullptr, *tndat = nullptr;
   int4* ptab = nullptr;  // per type pair: first row, NDAT, 1/bin bits, table present
   // FP32 path, tables on one grid (k_nonbonded_f32's UNI; NBArgs::tuni)
   uint2* pbase = nullptr;
@@ -138,7 +137,8 @@ struct DevList {
   float uinv = 0, r2_none = 0;
   int urows = 0;
   bool uni = false;
-  void *tbin = nullptr, *tinv = nullptr, *tfp = nullptr, *tx = nullptr;
+  void *tfp = nullptr, *tx = nullptr;  // FP32 path
+  double4* tcoef64 = nullptr;          // FP64 path (NBArgs::tcoef64)
   float4* tcoef = nullptr;  // FP32 path: per row {F - dF e, P - dP e, dF, dP} (NBArgs::tcoef)
   int ntab = 0, nrows = 0;
   bool use_smem = false;  // tables staged in shared memory (tuning)
@@ -378,13 +378,10 @@ void build_list(ibg_ctx* c, const ibg_desc* d, int which) {
   // without a table (it then stops the step with an error)
   while (xx.size() < 2) { fp.push_back(0); fp.push_back(0); xx.push_back(0); }
   L.nrows = (int)xx.size();
-  L.ltab = dupload(ltab, o);
-  L.toff = dupload(toff, o);
-  L.tndat = dupload(tnd, o);
   if (c->prec == IBG_PREC_FP32_FIXED) {
-    std::vector<float> f1(fp.begin(), fp.end()), x1(xx.begin(), xx.end()), b1(bin.begin(), bin.end()), i1(bin.size());
+    std::vector<float> f1(fp.begin(), fp.end()), x1(xx.begin(), xx.end()), i1(bin.size());
     for (size_t k = 0; k < bin.size(); ++k) i1[k] = (float)(1.0 / (double)(float)bin[k]);
-    L.tfp = dupload(f1, o); L.tx = dupload(x1, o); L.tbin = dupload(b1, o); L.tinv = dupload(i1, o);
+    L.tfp = dupload(f1, o); L.tx = dupload(x1, o);
     // interpolation coefficients of every row k of table t (local index n =
     // k - toff[t]): with u = r/bin - n, the kernel's alpha = (r - X_k)/bin
     // is u - e_k, e_k = X_k/bin - n, so F = F_k + (F_k+1 - F_k) alpha is
@@ -442,7 +439,28 @@ void build_list(ibg_ctx* c, const ibg_desc* d, int which) {
       L.pbase = dupload(pb, o);
     }
   } else {
-    L.tfp = dupload(fp, o); L.tx = dupload(xx, o); L.tbin = dupload(bin, o);
+    // the same coefficients in FP64, from the table rows: F = A + B u, P = C + D
+    // u with u = r/bin - n
+    std::vector<double4> co(L.nrows);
+    for (auto& r : co) r.x = r.y = r.z = r.w = 0.0;
+    std::vector<int4> pt((size_t)NT * NT);
+    for (int t = 0; t < L.ntab; ++t)
+      for (int k = toff[t]; k < toff[t + 1]; ++k) {
+        const bool last = k + 1 >= toff[t + 1];
+        const double fk = fp[2 * (size_t)k], pk = fp[2 * (size_t)k + 1];
+        const double df = last ? 0.0 : fp[2 * (size_t)k + 2] - fk, dp = last ? 0.0 : fp[2 * (size_t)k + 3] - pk;
+        const double e = xx[k] / bin[t] - (double)(k - toff[t]);
+        co[k].x = fk - df * e; co[k].y = pk - dp * e; co[k].z = df; co[k].w = dp;
+      }
+    L.tcoef64 = dupload(co, o);
+    for (size_t k = 0; k < pt.size(); ++k) {
+      const int t = ltab[k];
+      const double inv = t >= 0 ? 1.0 / bin[t] : 0.0;
+      int ib[2];
+      std::memcpy(ib, &inv, sizeof(inv));
+      pt[k] = t >= 0 ? make_int4(toff[t], tnd[t], ib[0], ib[1]) : make_int4(-1, 0, 0, 0);
+    }
+    L.ptab = dupload(pt, o);
   }
   // launch default: tables read through L1 (staged, the FP64 kernel's launch on
   // the 40,000-bead melt takes 82 us instead of 59)
@@ -541,9 +559,8 @@ void make_args(ibg_ctx* c) {
     n.pos4 = L.pos4; n.posq = L.posq; n.counts = L.counts; n.slice_w = L.slice_w; n.entries = L.entries;
     n.w_cap = L.w_cap; n.work = w;
     n.fsort = (acc_t*)L.fsort;
-    n.ltab = L.ltab; n.toff = L.toff; n.tndat = L.tndat; n.tbin = (const R*)L.tbin; n.tinv = (const R*)L.tinv;
-    n.tfp = (const R*)L.tfp; n.tx = (const R*)L.tx; n.ptab = L.ptab; n.chunk = c->nb_chunk;
-    n.tcoef = L.tcoef; n.pbase = L.pbase; n.tuni = L.tuni; n.uinv = L.uinv; n.r2_none = L.r2_none; n.urows = L.urows;
+    n.tfp = (const R*)L.tfp; n.tx = (const R*)L.tx; n.ptab = L.ptab; n.chunk = sizeof(R) == 4 ? c->nb_chunk : 24;  // the FP64 path has no choice of it
+    n.tcoef = L.tcoef; n.tcoef64 = L.tcoef64; n.pbase = L.pbase; n.tuni = L.tuni; n.uinv = L.uinv; n.r2_none = L.r2_none; n.urows = L.urows;
     n.rows = c->nb_rows;
     n.window = c->nb_window;
     n.ntab = L.ntab; n.nrows = L.nrows; n.rcutsq = (R)L.rcutsq;
@@ -715,23 +732,20 @@ template <>
 NBKernel<float, true> nb_kernel<float, true>(const NBKey& k) { return nb_kernel_b<true>(k); }
 template <>
 NBKernel<double, false> nb_kernel<double, false>(const NBKey& k) {
-  return k.smem ? k_nonbonded<double, true, 8, false> : k_nonbonded<double, false, 8, false>;
+  return k.smem ? k_nonbonded<true, 8, false> : k_nonbonded<false, 8, false>;
 }
 template <>
 NBKernel<double, true> nb_kernel<double, true>(const NBKey& k) {
-  return k.smem ? k_nonbonded<double, true, 8, true> : k_nonbonded<double, false, 8, true>;
+  return k.smem ? k_nonbonded<true, 8, true> : k_nonbonded<false, 8, true>;
 }
 
 // Dynamic shared memory of a nonbonded launch over list L: the sums, and the
 // tables when they are staged (smem_limit: the most a launch may ask for).
 constexpr size_t kSmemLimit = 200 * 1024;
 size_t nb_smem_of(const ibg_ctx* c, const DevList& L, const NBKey& k, bool staged) {
-  if (c->prec != IBG_PREC_FP32_FIXED) {
-    const size_t rs = sizeof(double);
-    return staged ? 9 * 256 * sizeof(double) + rs * 3 * (size_t)L.nrows + 2 * rs * L.ntab +
-                        sizeof(int) * ((size_t)c->ntype * c->ntype + 2 * L.ntab + 1) + 64
-                  : 9 * 9 * sizeof(double);
-  }
+  if (c->prec != IBG_PREC_FP32_FIXED)
+    return 96 * sizeof(double) +
+           (staged ? sizeof(double4) * (size_t)L.nrows + sizeof(int4) * (size_t)c->ntype * c->ntype : 0);
   size_t b = (size_t)nb_acc_bytes(L.mixed, k.nt);
   if (staged) {
     b += sizeof(int4) * (size_t)c->ntype * c->ntype + 64;

@@ -1385,14 +1385,9 @@ struct NBArgs {
   int w_cap;                       // rows of 32 entries per slice
   int work;                        // index of this launch's work counter
   typename Prec<R>::acc_t* fsort;  // per slot, in blocks of 32 slots (fs_at)
-  // tables of this list: ltab[ti*ntype+tj] = local table or -1; rows of table
-  // t are [toff[t], toff[t+1]); fp = {F,P} per row, x = RNBOND per row
-  const int* ltab;
-  const int* toff;
-  const int* tndat;
-  const R* tbin;
-  const R* tinv; // 1/bin per table (FP32 force kernel)
-  const int4* ptab;  // FP32 kernel: per type pair {first row, NDAT, 1/bin bits, 1 if a table}
+  // tables of this list, per type pair: FP32 path {first row, NDAT, 1/bin bits,
+  // 1 if a table}, FP64 path {first row or -1, NDAT, 1/bin low and high word}
+  const int4* ptab;
   // FP32 kernel, UNI (all tables on one grid, 1/bin = uinv): the table numbers
   // per type, a byte per type of the neighbour, and the coefficient rows of
   // every table one after another, urows each, F scaled by -2^32; the last of
@@ -1401,8 +1396,8 @@ struct NBArgs {
   const float4* tuni;
   float uinv, r2_none;
   int urows;
-  int chunk;         // FP32 kernel: 256ths of the units taken dynamically after the blocks' own ranges (0: all, per warp)
-  int window;        // FP32 kernel, chunk > 0: 0 = each block one contiguous range of units; W > 0 = runs of W
+  int chunk;         // 256ths of the units taken dynamically after the blocks' own ranges (0: all, per warp)
+  int window;        // chunk > 0: 0 = each block one contiguous range of units; W > 0 = runs of W
                      // consecutive units dealt to the blocks in turn (block b takes runs b, b + G, b + 2G, ...)
   int rows;          // list rows per work unit, a multiple of kEnergyRows
   // FP32 kernel: pairs whose r^2 lies within a relative 1e-6 of the cutoff
@@ -1416,10 +1411,11 @@ struct NBArgs {
   const int* idx;
   const double* S;
   int natoms;
-  const R* tfp;  // 2 per row
+  const R* tfp;  // FP32 path: {F, P} per row, and X = RNBOND per row (k_nb_near)
   // FP32 kernel: per row {A, C, B, D}, -2^32 F = A + B u and P = C + D u with
   // u = r/bin - (row within the table); one 16-byte read per pair
   const float4* tcoef;
+  const double4* tcoef64;  // FP64 kernel: the same unscaled, in FP64
   const R* tx;
   int ntab, nrows;
   R rcutsq;
@@ -1446,178 +1442,7 @@ __device__ __forceinline__ int nb_units_per_slice(const NBArgs<R>& A) {
   return max(1, (min(A.sc->rows_max[A.work], A.w_cap) + A.rows - 1) / A.rows);
 }
 
-// NONBONDED_FORCE.F90:45-104.  Persistent grid; a warp owns one slice of
-// P = 32/T slots at a time and T lanes walk each slot's list; list reads are
-// coalesced 128-byte rows, neighbour positions are float4 gathers from the
-// cell-ordered array.  i-forces are summed in registers and reduced exactly
-// over the slot's lanes (integer shuffles); j-forces are 64-bit integer
-// atomics.  Tables are staged in shared memory when SMEM.
-template <typename R, bool SMEM, int T, bool B>
-__global__ void __launch_bounds__(256, 4) k_nonbonded(__grid_constant__ const NBArgs<R> A0, const NBArgs<R>* const* tab,
-                                                      const BlockMap bm) {
-  using P = Prec<R>;
-  pdl_wait();
-  pdl_trigger();
-  const Blk bk = blk<B>(bm);
-  __shared__ NBArgs<R> s_args;
-  if (B) stage_args(&s_args, tab[bk.sys]);
-  const NBArgs<R>& A = B ? s_args : A0;
-  Scalars* sc = A.sc;
-  if (nb_idle(A)) return;
-  using PT = typename P::pos_t;
-  using reg_t = typename P::reg_t;
-  constexpr int PS = 32 / T;
-  extern __shared__ unsigned char smem_raw[];
-  const int* ltab = A.ltab;
-  const int* toff = A.toff;
-  const int* tndat = A.tndat;
-  const R* tbin = A.tbin;
-  const R* tfp = A.tfp;
-  const R* tx = A.tx;
-  double* red = (double*)smem_raw;  // 9 * 9 doubles
-  if (SMEM) {
-    unsigned char* p = smem_raw + 9 * 9 * sizeof(double);
-    R* s_fp = (R*)p;               p += sizeof(R) * 2 * A.nrows;
-    R* s_x = (R*)p;                p += sizeof(R) * A.nrows;
-    R* s_bin = (R*)p;              p += sizeof(R) * A.ntab;
-    int* s_ltab = (int*)p;         p += sizeof(int) * A.ntype * A.ntype;
-    int* s_toff = (int*)p;         p += sizeof(int) * (A.ntab + 1);
-    int* s_ndat = (int*)p;
-    for (int k = threadIdx.x; k < 2 * A.nrows; k += blockDim.x) s_fp[k] = A.tfp[k];
-    for (int k = threadIdx.x; k < A.nrows; k += blockDim.x) s_x[k] = A.tx[k];
-    for (int k = threadIdx.x; k < A.ntab; k += blockDim.x) { s_bin[k] = A.tbin[k]; s_ndat[k] = A.tndat[k]; }
-    for (int k = threadIdx.x; k < A.ntype * A.ntype; k += blockDim.x) s_ltab[k] = A.ltab[k];
-    for (int k = threadIdx.x; k <= A.ntab; k += blockDim.x) s_toff[k] = A.toff[k];
-    __syncthreads();
-    ltab = s_ltab; toff = s_toff; tndat = s_ndat; tbin = s_bin; tfp = s_fp; tx = s_x;
-  }
-  R b[3], bi[3], b2[3];
-  box_of<R>(sc, b, bi, b2);
-  const PT* pos = (const PT*)A.pos4;
-  const int lane = threadIdx.x & 31, grp = lane / T, q = lane % T;
-  double acc[9];
-#pragma unroll
-  for (int k = 0; k < 9; ++k) acc[k] = 0.0;
-  unsigned err = 0;
-  const bool run = true;
-  // work unit = up to ROWS rows of 32 entries of one slice; units are taken
-  // dynamically so that warps finish within one unit of each other
-  const int ROWS = A.rows;
-  const int U = nb_units_per_slice(A);
-  const int nunits = A.nslices * U;
-  for (;;) {
-    int u = 0;
-    if (lane == 0) u = run ? (int)atomicAdd(&sc->work[A.work], 1u) : nunits;
-    u = __shfl_sync(0xffffffffu, u, 0);
-    if (u >= nunits) break;
-    const int g = u / U;
-    const int r0 = (u - g * U) * ROWS;
-    const int w = min(A.slice_w[g], A.w_cap);
-    if (r0 >= w) continue;
-    const int r1 = min(w, r0 + ROWS);
-    const int s = g * PS + grp;
-    const bool valid = s < A.n;
-    const int cnt = valid ? A.counts[s] : 0;
-    const int* ent = A.entries + (long long)g * A.w_cap * 32 + lane;
-    PT pi;
-    if (valid) pi = pos[s];
-    else { pi.x = pi.y = pi.z = 0; pi.w = P::tbits(0); }
-    const int wi = P::bits(pi.w);
-    const int ti = wi & 0xffff, li = wi >> 16;
-    reg_t fi0 = 0, fi1 = 0, fi2 = 0;
-    auto pair = [&](int t, const PT& pj) {
-      R d0 = pi.x - pj.x, d1 = pi.y - pj.y, d2 = pi.z - pj.z;
-      d0 = d0 - r_round(d0 * bi[0]) * b[0];
-      d1 = d1 - r_round(d1 * bi[1]) * b[1];
-      d2 = d2 - r_round(d2 * bi[2]) * b[2];
-      R r2 = d0 * d0;
-      r2 = r2 + d1 * d1;
-      r2 = r2 + d2 * d2;
-      if (!(r2 < A.rcutsq)) return;
-      const int wj = P::bits(pj.w);
-      const int tj = wj & 0xffff, lj = wj >> 16;
-      const int tab = ltab[ti * A.ntype + tj];
-      if (tab < 0) { err |= EB_MISSING_TABLE; return; }
-      const R r = r_sqrt(r2);
-      const R bin = tbin[tab];
-      const int ni = fint(r / bin);
-      if (ni < 0 || ni > tndat[tab]) { err |= EB_TABLE_RANGE; return; }
-      const int row = toff[tab] + ni;
-      const R alpha = (r - tx[row]) / bin;
-      const R f0 = tfp[2 * row], p0 = tfp[2 * row + 1], f1 = tfp[2 * row + 2], p1 = tfp[2 * row + 3];
-      const R one_a = (R)1.0 - alpha;
-      const R fij = f0 * one_a + f1 * alpha;
-      const R vij = p0 * one_a + p1 * alpha;
-      if (li == 1) acc[0] += (double)vij;
-      else if (li == 2) {
-        if (lj == 2) acc[1] += (double)vij;
-        else if (lj == 3) acc[2] += (double)vij;
-      } else if (li == 3) acc[2] += (double)vij;
-      const R fx = fij * d0, fy = fij * d1, fz = fij * d2;
-      const reg_t qx = P::q(fx, &sc->err), qy = P::q(fy, &sc->err), qz = P::q(fz, &sc->err);
-      fi0 += qx; fi1 += qy; fi2 += qz;
-      typename P::acc_t* fj = A.fsort + fs_at(t);
-      P::add(fj, -qx);
-      P::add(fj + 32, -qy);
-      P::add(fj + 64, -qz);
-      acc[3] += (double)(fx * d0);
-      acc[4] += (double)(fy * d1);
-      acc[5] += (double)(fz * d2);
-      acc[6] += (double)(fy * d0);
-      acc[7] += (double)(fz * d0);
-      acc[8] += (double)(fz * d1);
-    };
-    // two rows per iteration: both entry loads and both position gathers are
-    // in flight before either pair is evaluated
-    for (int it = r0; it < r1; it += 2) {
-      const bool v0 = it * T + q < cnt;
-      const bool v1 = it + 1 < r1 && (it + 1) * T + q < cnt;
-      const int t0 = v0 ? __ldcs(ent + it * 32) : 0;
-      const int t1 = v1 ? __ldcs(ent + (it + 1) * 32) : 0;
-      const PT p0 = pos[t0];
-      const PT p1 = pos[t1];
-      if (v0) pair(t0, p0);
-      if (v1) pair(t1, p1);
-    }
-#pragma unroll
-    for (int o = T / 2; o > 0; o >>= 1) {
-      fi0 += __shfl_down_sync(0xffffffffu, fi0, o, T);
-      fi1 += __shfl_down_sync(0xffffffffu, fi1, o, T);
-      fi2 += __shfl_down_sync(0xffffffffu, fi2, o, T);
-    }
-    if (q == 0 && valid && r0 * T < cnt) {
-      typename P::acc_t* fo = A.fsort + fs_at(s);
-      P::add(fo, fi0);
-      P::add(fo + 32, fi1);
-      P::add(fo + 64, fi2);
-    }
-  }
-  if (err) atomicOr(&sc->err, err);
-  __syncthreads();
-  block_sums<9>(acc, red);
-  if (threadIdx.x < 9) atomicAdd((double*)&sc->nbacc[A.work][threadIdx.x], red[threadIdx.x]);
-}
-
-// round(v * 2^S) to the nearest 64-bit integer: the scaling by a power of two
-// is exact and the conversion rounds to nearest.  Values of magnitude
-// 2^(63-S) and above (and Inf/NaN) raise EB_FIXED and count as 0.
-// fabsf(fij) r below 0.99 kFixMax, tested on the force scaled by 2^32
-constexpr float kFixLimScaled = 0.99f * kFixMax * kFixScale;
-// The FP32 nonbonded kernels' energy and virial sums, at the start of their
-// dynamic shared memory: 7 per lane of their 256-thread blocks for a list of
-// one label, 9 for a list of several.  A lane adds to its own words, with no
-// shuffle and no half-idle warp (per pair of lanes, they took 16 shuffles and
-// nine half-warp updates for every eight list rows).
-__host__ __device__ constexpr int nb_acc_bytes(bool mixed, int nt) { return (mixed ? 9 : 7) * nt * (int)sizeof(long long); }
-
-template <int S>
-__device__ __forceinline__ long long fixq(float v, unsigned& err) {
-  const float s = v * (float)(1ull << S);
-  if (!(fabsf(s) < 0x1p63f)) { err |= EB_FIXED; return 0; }
-  return __float2ll_rn(s);
-}
-
-// The sequence of work units one warp of an FP32 nonbonded launch takes
+// The sequence of work units one warp of a nonbonded launch takes
 // (NBArgs::chunk, NBArgs::window): first units of its block's share, taken
 // through a shared counter -- a contiguous range of units (neighbouring
 // slices), or with a window runs of W consecutive units dealt to the blocks in
@@ -1625,13 +1450,14 @@ __device__ __forceinline__ long long fixq(float v, unsigned& err) {
 // it in L1, with no barrier between them; then the last chunk/256 of all units (all of them with chunk 0),
 // taken from a global counter by whichever warps get there first.  A warp
 // knows its next unit while it still works on one, so that it can load ahead.
+template <typename R>
 struct NbUnits {
-  const NBArgs<float>& A;
+  const NBArgs<R>& A;
   const Blk& bk;
   int* own;  // the block's counter, in shared memory
   int U;     // units per slice
   int lo, hi;
-  __device__ __forceinline__ NbUnits(const NBArgs<float>& A_, const Blk& bk_, int U_, int* own_)
+  __device__ __forceinline__ NbUnits(const NBArgs<R>& A_, const Blk& bk_, int U_, int* own_)
       : A(A_), bk(bk_), own(own_), U(U_) {
     const int ns = nstat();
     lo = A.window > 0 ? 0 : (int)((long long)ns * bk.b / bk.g);
@@ -1658,6 +1484,207 @@ struct NbUnits {
     return u < A.nslices * U ? u : -1;
   }
 };
+
+// NONBONDED_FORCE.F90:45-104, FP64 path.  Persistent grid; a warp owns one
+// slice of P = 32/T slots at a time and T lanes walk each slot's list; list
+// reads are coalesced 128-byte rows, neighbour positions are 32-byte gathers
+// from the cell-ordered array.  i-forces are summed in registers and reduced
+// over the slot's lanes; j-forces are FP64 atomics.  Tables are staged in
+// shared memory when SMEM.
+//
+// Bound by FP64 issue and by the latency of its gathers.  A pair cost two FP64
+// divisions, three roundings to the nearest image and seven table reads; it
+// now multiplies by 1/bin, picks the image by comparison, and reads a row of
+// coefficients (A + B u, C + D u); two rows are evaluated in step and units are
+// handed out as in k_nonbonded_f32.  16 warps per SM at 128 registers: at 24
+// warps (80 registers, 108 bytes of spills) the launch took 189 us on the
+// 160,000-bead melt, with 16 174 (before: 216), without the block ranges.
+template <bool SMEM, int T, bool B>
+__global__ void __launch_bounds__(256, 2) k_nonbonded(__grid_constant__ const NBArgs<double> A0,
+                                                      const NBArgs<double>* const* tab, const BlockMap bm) {
+  using P = Prec<double>;
+  pdl_wait();
+  pdl_trigger();
+  const Blk bk = blk<B>(bm);
+  __shared__ NBArgs<double> s_args;
+  if (B) stage_args(&s_args, tab[bk.sys]);
+  const NBArgs<double>& A = B ? s_args : A0;
+  Scalars* sc = A.sc;
+  if (nb_idle(A)) return;
+  constexpr int PS = 32 / T;
+  extern __shared__ unsigned char smem_raw[];
+  double* red = (double*)smem_raw;  // 9 * 9 doubles
+  const int4* ptab = A.ptab;        // per type pair {first row or -1, NDAT, 1/bin}
+  const double4* tco = A.tcoef64;
+  if (SMEM) {
+    double4* s_co = (double4*)(smem_raw + 96 * sizeof(double));
+    int4* s_ptab = (int4*)(s_co + A.nrows);
+    for (int k = threadIdx.x; k < A.nrows; k += blockDim.x) s_co[k] = A.tcoef64[k];
+    for (int k = threadIdx.x; k < A.ntype * A.ntype; k += blockDim.x) s_ptab[k] = A.ptab[k];
+    __syncthreads();
+    ptab = s_ptab; tco = s_co;
+  }
+  double b[3], bi[3], b2[3];
+  box_of<double>(sc, b, bi, b2);
+  const double4* pos = (const double4*)A.pos4;
+  const int lane = threadIdx.x & 31, grp = lane / T, q = lane % T;
+  double acc[9];
+#pragma unroll
+  for (int k = 0; k < 9; ++k) acc[k] = 0.0;
+  unsigned err = 0;
+  // a work unit is `rows` rows of 32 entries of one slice; the next one's
+  // header is loaded while the warp works on this one
+  const int rows = A.rows;
+  const int U = nb_units_per_slice(A);
+  struct Head {
+    int u, w, cnt;
+  };
+  auto head = [&](int u) {
+    const int g = U == 1 ? u : u / U;
+    const int s = g * PS + grp;
+    return Head{u, min(A.slice_w[g], A.w_cap), s < A.n ? A.counts[s] : 0};
+  };
+  __shared__ int s_next;
+  if (threadIdx.x == 0) s_next = 0;
+  __syncthreads();
+  NbUnits<double> seq(A, bk, U, &s_next);
+  struct Geo {
+    double d0, d1, d2, r2;
+  };
+  auto unit = [&](const Head& h) {
+    const int g = U == 1 ? h.u : h.u / U;
+    const int r0 = (h.u - g * U) * rows, r1 = min(h.w, r0 + rows);
+    if (r0 >= r1) return;
+    const int s = g * PS + grp;
+    // the lane's entries, T per row; a lane without one reads slot 0, which
+    // then does not count
+    int left = min(h.cnt, r1 * T) - r0 * T - q;
+    const bool mine = left > 0;
+    const int* e = A.entries + (size_t)g * ((unsigned)A.w_cap * 32u) + (unsigned)(r0 * 32 + lane);
+    int t0 = left > 0 ? __ldcs(e) : 0, t1 = left > T ? __ldcs(e + 32) : 0;
+    double4 pi;
+    if (s < A.n) pi = pos[s];
+    else { pi.x = pi.y = pi.z = 0; pi.w = P::tbits(0); }
+    const int wi = P::bits(pi.w);
+    const int ti = wi & 0xffff, li = wi >> 16;
+    const int4* pti = ptab + ti * A.ntype;
+    double fi0 = 0, fi1 = 0, fi2 = 0;
+    // the nearest image: d - ANINT(d/L) L of two positions inside the box
+    // (they could choose differently only at |d| = L/2, beyond the cutoff)
+    auto image = [](double d, double L, double half) {
+      return d > half ? d - L : (d < -half ? d + L : d);
+    };
+    auto geo = [&](const double4& pj) {
+      Geo G;
+      G.d0 = image(pi.x - pj.x, b[0], b2[0]);
+      G.d1 = image(pi.y - pj.y, b[1], b2[1]);
+      G.d2 = image(pi.z - pj.z, b[2], b2[2]);
+      G.r2 = G.d0 * G.d0;
+      G.r2 = G.r2 + G.d1 * G.d1;
+      G.r2 = G.r2 + G.d2 * G.d2;
+      return G;
+    };
+    // a pair's row and weight; clears `in` (and notes the error) where it has
+    // no table or lies beyond it
+    auto look = [&](const Geo& G, bool& in, int wj, double& u) {
+      const int4 pt = pti[wj & 0xffff];
+      const double r = r_sqrt(in ? G.r2 : 1.0);
+      const double rb = r * __hiloint2double(pt.w, pt.z);
+      const int ni = fint(rb);
+      u = rb - (double)ni;
+      if (in && pt.x < 0) { err |= EB_MISSING_TABLE; in = false; }
+      if (in && (ni < 0 || ni > pt.y)) { err |= EB_TABLE_RANGE; in = false; }
+      return in ? pt.x + ni : 0;
+    };
+    auto pair = [&](const Geo& G, int t, int wj, const double4& co, double u) {
+      const double fij = co.x + co.z * u, vij = co.y + co.w * u;
+      const int lj = wj >> 16;
+      if (li == 1) acc[0] += vij;
+      else if (li == 2) {
+        if (lj == 2) acc[1] += vij;
+        else if (lj == 3) acc[2] += vij;
+      } else if (li == 3) acc[2] += vij;
+      const double fx = fij * G.d0, fy = fij * G.d1, fz = fij * G.d2;
+      fi0 += fx; fi1 += fy; fi2 += fz;
+      double* fj = A.fsort + fs_at(t);
+      P::add(fj, -fx);
+      P::add(fj + 32, -fy);
+      P::add(fj + 64, -fz);
+      acc[3] += fx * G.d0;
+      acc[4] += fy * G.d1;
+      acc[5] += fz * G.d2;
+      acc[6] += fy * G.d0;
+      acc[7] += fz * G.d0;
+      acc[8] += fz * G.d1;
+    };
+    for (int it = r0; it < r1; it += 2) {
+      const double4 p0 = pos[(unsigned)t0];
+      const double4 p1 = pos[(unsigned)t1];
+      const bool v0 = left > 0, v1 = left > T;
+      left -= 2 * T;
+      e += 64;
+      const int n0 = left > 0 ? __ldcs(e) : 0;
+      const int n1 = left > T ? __ldcs(e + 32) : 0;
+      const Geo g0 = geo(p0), g1 = geo(p1);
+      bool in0 = v0 && g0.r2 < A.rcutsq, in1 = v1 && g1.r2 < A.rcutsq;
+      if (in0 || in1) {
+        const int w0 = P::bits(p0.w), w1 = P::bits(p1.w);
+        double u0, u1;
+        const int k0 = look(g0, in0, w0, u0), k1 = look(g1, in1, w1, u1);
+        const double4 c0 = tco[k0], c1 = tco[k1];
+        if (in0) pair(g0, t0, w0, c0, u0);
+        if (in1) pair(g1, t1, w1, c1, u1);
+      }
+      t0 = n0;
+      t1 = n1;
+    }
+#pragma unroll
+    for (int o = T / 2; o > 0; o >>= 1) {
+      fi0 += __shfl_down_sync(0xffffffffu, fi0, o, T);
+      fi1 += __shfl_down_sync(0xffffffffu, fi1, o, T);
+      fi2 += __shfl_down_sync(0xffffffffu, fi2, o, T);
+    }
+    if (q == 0 && mine) {
+      double* fo = A.fsort + fs_at(s);
+      P::add(fo, fi0);
+      P::add(fo + 32, fi1);
+      P::add(fo + 64, fi2);
+    }
+  };
+  int u = seq.next();
+  Head h{-1, 0, 0};
+  if (u >= 0) h = head(u);
+  while (h.u >= 0) {
+    u = seq.next();
+    Head hn{-1, 0, 0};
+    if (u >= 0) hn = head(u);
+    unit(h);
+    h = hn;
+  }
+  if (err) atomicOr(&sc->err, err);
+  __syncthreads();
+  block_sums<9>(acc, red);
+  if (threadIdx.x < 9) atomicAdd((double*)&sc->nbacc[A.work][threadIdx.x], red[threadIdx.x]);
+}
+
+// round(v * 2^S) to the nearest 64-bit integer: the scaling by a power of two
+// is exact and the conversion rounds to nearest.  Values of magnitude
+// 2^(63-S) and above (and Inf/NaN) raise EB_FIXED and count as 0.
+// fabsf(fij) r below 0.99 kFixMax, tested on the force scaled by 2^32
+constexpr float kFixLimScaled = 0.99f * kFixMax * kFixScale;
+// The FP32 nonbonded kernels' energy and virial sums, at the start of their
+// dynamic shared memory: 7 per lane of their 256-thread blocks for a list of
+// one label, 9 for a list of several.  A lane adds to its own words, with no
+// shuffle and no half-idle warp (per pair of lanes, they took 16 shuffles and
+// nine half-warp updates for every eight list rows).
+__host__ __device__ constexpr int nb_acc_bytes(bool mixed, int nt) { return (mixed ? 9 : 7) * nt * (int)sizeof(long long); }
+
+template <int S>
+__device__ __forceinline__ long long fixq(float v, unsigned& err) {
+  const float s = v * (float)(1ull << S);
+  if (!(fabsf(s) < 0x1p63f)) { err |= EB_FIXED; return 0; }
+  return __float2ll_rn(s);
+}
 
 // 1/sqrt(x) of a normal x (squared distances are far above the denormals), as
 // rsqrtf gives it there, without rsqrtf's scaling of denormals.
@@ -1963,7 +1990,7 @@ __global__ void __launch_bounds__(NT, 1024 / NT) k_nonbonded_f32(__grid_constant
       atomicAdd(fo + 64, (unsigned long long)fi2);
     }
   };
-  NbUnits seq(A, bk, U, &s_next);
+  NbUnits<float> seq(A, bk, U, &s_next);
   int u = seq.next();
   Head h{-1, 0, 0};
   if (u >= 0) h = head(u);
@@ -2172,7 +2199,7 @@ __global__ void __launch_bounds__(256, 3) k_nonbonded_slices(__grid_constant__ c
   __shared__ int s_next;
   if (threadIdx.x == 0) s_next = 0;
   __syncthreads();
-  NbUnits seq(A, bk, U, &s_next);
+  NbUnits<float> seq(A, bk, U, &s_next);
   for (int u = seq.next(); u >= 0; u = seq.next()) unit(u);
   if (err) atomicOr(&sc->err, err);
   nb_block_sums<NE, 256>(A, lacc);
