@@ -181,6 +181,7 @@ template <typename R, bool B>
 __global__ void k_positions(__grid_constant__ const PosArgs a0, const PosArgs* const* tab, const BlockMap bm,
                             int begin) {
   using PT = typename Prec<R>::pos_t;
+  pdl_wait();
   pdl_trigger();
   const Blk bk = blk<B>(bm);
   const PosArgs& a = B ? *tab[bk.sys] : a0;
@@ -2995,6 +2996,7 @@ __device__ double wsum(const double* p, int g) {
 template <bool B>
 __global__ void k_finalize(__grid_constant__ const FinalArgs F0, const FinalArgs* const* tab, const BlockMap bm) {
   pdl_wait();
+  pdl_trigger();
   const Blk bk = blk<B>(bm);
   const FinalArgs& F = B ? *tab[bk.sys] : F0;
   Scalars* sc = F.sc;
