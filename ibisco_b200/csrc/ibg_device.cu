@@ -978,13 +978,11 @@ constexpr size_t kMaxChains = 32;
 // The system runs steps step_before+1 .. last; observables of step k go to
 // ring slot k - base.
 // Step counter, ring base and step limit for the next run, in stream order
-// on the context's stream (sync: also wait for it, for launches on another
-// stream).
-void set_step_counter(ibg_ctx* c, int step_before, int base, int last, bool sync) {
+// on the context's stream.
+void set_step_counter(ibg_ctx* c, int step_before, int base, int last) {
   k_set_counter<<<1, 1, 0, c->st>>>(c->sc, step_before, base, last);
   CK(cudaGetLastError());
   ++c->launches;
-  if (sync) CK(cudaStreamSynchronize(c->st));
 }
 
 int check_bits(ibg_ctx* c, unsigned bits);
@@ -1020,15 +1018,6 @@ void obs_to_c(const ObsD& o, ibg_obs* out) {
   out->cell_clamps = o.cell_clamps;
   out->step = o.step;
   out->status = o.status;
-}
-
-int read_obs(ibg_ctx* c, ibg_obs* out) {
-  if (!out) return IBG_OK;
-  ObsD o;
-  CK(cudaMemcpyAsync(&o, &c->sc->obs, sizeof(ObsD), cudaMemcpyDeviceToHost, c->st));
-  CK(cudaStreamSynchronize(c->st));
-  obs_to_c(o, out);
-  return IBG_OK;
 }
 
 // A list build that outgrew its slices raised the abort flag (the remaining
@@ -1109,6 +1098,7 @@ int ibg_set_list_rows(ibg_ctx* c, int rows) {
       L.w_cap = rows;
     }
     refresh_args(c);
+    CK(cudaStreamSynchronize(c->st));  // a batch reads the arguments on its own stream
     drop_graphs(c);
   } catch (CudaError& e) {
     return fail(c, IBG_E_CUDA, cudaGetErrorString(e.e));
@@ -1723,7 +1713,7 @@ static int run_steps(ibg_ctx* c, int first, int nsteps, ibg_obs* per_step, bool 
     int done = 0;
     float run_ms_total = 0.f;
     for (int attempt = 0; attempt < 8 && done < nsteps; ++attempt) {
-      set_step_counter(c, first + done - 1, first, first + nsteps - 1, false);
+      set_step_counter(c, first + done - 1, first, first + nsteps - 1);
       if (c->flush_bytes) {
         if (!c->flush_buf) CK(cudaMalloc(&c->flush_buf, c->flush_bytes));
         while ((int)c->step_ev.size() < 2 * nsteps) {
@@ -2060,6 +2050,9 @@ struct ibg_batch {
   cudaEvent_t fork_ev[2] = {nullptr, nullptr}, run_ev[2] = {nullptr, nullptr};
   // per-system pointers to the argument blocks, by kind
   void** t_pos = nullptr;
+  Scalars** t_sc = nullptr;       // every system's scalars
+  BatchStat* stat = nullptr;      // k_batch_stat's output, and the host's page-locked copy
+  BatchStat* hstat = nullptr;
   void** t_list[2] = {nullptr, nullptr};
   void** t_nb[2] = {nullptr, nullptr};
   void** t_col[2] = {nullptr, nullptr};
@@ -2333,10 +2326,16 @@ int ibg_batch_create(ibg_ctx* const* ctxs, int n, ibg_batch** out) {
     }
     if (b->prec == IBG_PREC_FP32_FIXED) batch_layout<float>(b.get());
     else batch_layout<double>(b.get());
+    std::vector<Scalars*> scs;
+    for (ibg_ctx* c : b->sys) scs.push_back(c->sc);
+    b->t_sc = dupload(scs, b->owned);
+    b->stat = dalloc<BatchStat>(n, b->owned);
+    CK(cudaHostAlloc(&b->hstat, sizeof(BatchStat) * (size_t)n, cudaHostAllocDefault));
     for (ibg_ctx* c : b->sys) c->in_batch = true;
     CK(cudaDeviceSynchronize());
   } catch (CudaError& e) {
     b->owned.free_all();
+    if (b->hstat) cudaFreeHost(b->hstat);
     return IBG_E_CUDA;
   }
   *out = b.release();
@@ -2354,12 +2353,27 @@ int ibg_batch_run(ibg_batch* b, int nsteps, const int* last_step, ibg_obs* last_
       last[s] = c->step_now + nsteps;
       if (last_step) last[s] = std::max(c->step_now, std::min(last[s], last_step[s]));
     }
+    // every system's status and observables in one copy (one read each of the
+    // flags, the errors and the observables cost ~30 us a system and run)
+    auto read_back = [&] {
+      k_batch_stat<<<(unsigned)n, 32, 0, b->st>>>(b->t_sc, b->stat);
+      CK(cudaGetLastError());
+      ++b->launches;
+      CK(cudaMemcpyAsync(b->hstat, b->stat, sizeof(BatchStat) * n, cudaMemcpyDeviceToHost, b->st));
+      CK(cudaStreamSynchronize(b->st));
+    };
+    bool have = false;
     float total_ms = 0.f;
     for (int attempt = 0; attempt < 8; ++attempt) {
       int need = 0;
       for (size_t s = 0; s < n; ++s) need = std::max(need, last[s] - from[s]);
       if (need == 0) break;
-      for (size_t s = 0; s < n; ++s) set_step_counter(b->sys[s], from[s], INT_MAX, last[s], true);
+      // on the batch's stream: the contexts' own streams are idle between calls
+      for (size_t s = 0; s < n; ++s) {
+        k_set_counter<<<1, 1, 0, b->st>>>(b->sys[s]->sc, from[s], INT_MAX, last[s]);
+        ++b->sys[s]->launches;
+      }
+      CK(cudaGetLastError());
       CK(cudaEventRecord(b->run_ev[0], b->st));
       for (int k = 0; k < need; ++k) {
         const unsigned v = batch_variant(b, from, last, k);
@@ -2381,7 +2395,8 @@ int ibg_batch_run(ibg_batch* b, int nsteps, const int* last_step, ibg_obs* last_
         b->launches += b->launches_per_variant[v & 7];
       }
       CK(cudaEventRecord(b->run_ev[1], b->st));
-      CK(cudaStreamSynchronize(b->st));
+      read_back();
+      have = true;
       float ms = 0.f;
       CK(cudaEventElapsedTime(&ms, b->run_ev[0], b->run_ev[1]));
       total_ms += ms;
@@ -2390,10 +2405,8 @@ int ibg_batch_run(ibg_batch* b, int nsteps, const int* last_step, ibg_obs* last_
       bool again = false;
       for (size_t s = 0; s < n; ++s) {
         ibg_ctx* c = b->sys[s];
-        if (grow_lists(c)) {
-          int st = 0;
-          CK(cudaMemcpy(&st, &c->sc->step, sizeof(int), cudaMemcpyDeviceToHost));
-          from[s] = st - 1;
+        if (b->hstat[s].abort && grow_lists(c)) {
+          from[s] = b->hstat[s].step - 1;
           again = true;
         } else {
           from[s] = last[s];
@@ -2402,6 +2415,7 @@ int ibg_batch_run(ibg_batch* b, int nsteps, const int* last_step, ibg_obs* last_
       if (!again) break;
     }
     b->run_ms = total_ms;
+    if (!have) read_back();
     // every system's status: a failing system does not hide the others'
     int first_rc = IBG_OK;
     for (size_t s = 0; s < n; ++s) {
@@ -2409,9 +2423,9 @@ int ibg_batch_run(ibg_batch* b, int nsteps, const int* last_step, ibg_obs* last_
       int rc = IBG_OK;
       if (from[s] < last[s]) rc = fail(c, IBG_E_CAPACITY, "neighbour-list storage could not be sized");
       c->step_now = from[s];
-      if (!rc) rc = check_device(c);
+      if (!rc) rc = check_bits(c, b->hstat[s].err);
       if (last_obs) {
-        read_obs(c, &last_obs[s]);
+        obs_to_c(b->hstat[s].obs, &last_obs[s]);
         last_obs[s].status = rc;
       }
       if (rc && !first_rc) {
@@ -2441,6 +2455,7 @@ void ibg_batch_destroy(ibg_batch* b) {
   cudaStreamSynchronize(b->st);
   for (auto& kv : b->graphs) cudaGraphExecDestroy(kv.second);
   b->owned.free_all();
+  if (b->hstat) cudaFreeHost(b->hstat);
   for (int k = 0; k < 2; ++k) {
     if (b->fork_ev[k]) cudaEventDestroy(b->fork_ev[k]);
     if (b->run_ev[k]) cudaEventDestroy(b->run_ev[k]);

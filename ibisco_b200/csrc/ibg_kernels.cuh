@@ -2307,9 +2307,8 @@ __global__ void __launch_bounds__(256) k_nb_near(__grid_constant__ const NBArgs<
     if (threadIdx.x == 0) near_overflow(sc, A.work, n);
     return;
   }
-  __shared__ unsigned long long s_sum[9];
-  if (threadIdx.x < 9) s_sum[threadIdx.x] = 0ull;
-  __syncthreads();
+  __shared__ long long red[9 + 9 * 8];
+  long long acc[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
   const float ux = (float)(sc->box[0] * 0x1p-32), uy = (float)(sc->box[1] * 0x1p-32), uz = (float)(sc->box[2] * 0x1p-32);
   unsigned err = 0;
   for (unsigned k = threadIdx.x; k < n; k += blockDim.x) {
@@ -2322,12 +2321,15 @@ __global__ void __launch_bounds__(256) k_nb_near(__grid_constant__ const NBArgs<
           atomicAdd(fsi + 32 * c, (unsigned long long)f);
           atomicAdd(fsj + 32 * c, (unsigned long long)(-f));
         },
-        [&](int t, long long e) { atomicAdd(&s_sum[t], (unsigned long long)e); });
+        [&](int t, long long e) {
+#pragma unroll
+          for (int c = 0; c < 9; ++c) acc[c] += c == t ? e : 0;
+        });
   }
   if (err) atomicOr(&sc->err, err);
-  __syncthreads();
-  if (threadIdx.x < 9 && s_sum[threadIdx.x] != 0)
-    atomicAdd(&sc->nbacc[A.work][threadIdx.x], s_sum[threadIdx.x]);
+  block_sums<9>(acc, red);
+  if (threadIdx.x < 9 && red[threadIdx.x] != 0)
+    atomicAdd(&sc->nbacc[A.work][threadIdx.x], (unsigned long long)red[threadIdx.x]);
   __syncthreads();
   if (threadIdx.x == 0) sc->near_n[A.work] = 0u;
 }
@@ -3123,6 +3125,24 @@ __global__ void k_set_counter(Scalars* sc, int step_before, int ring_base, int l
   sc->skip = 0;
   sc->stop_at = last;
   sc->done = step_before >= last ? 1 : 0;
+}
+
+// What the host reads after a batch's run, of every system in one copy.
+struct BatchStat {
+  int abort, step;
+  unsigned err, pad;
+  ObsD obs;
+};
+__global__ void k_batch_stat(const Scalars* const* scs, BatchStat* out) {
+  const Scalars* sc = scs[blockIdx.x];
+  BatchStat& o = out[blockIdx.x];
+  for (int k = threadIdx.x; k < (int)(sizeof(ObsD) / 8); k += blockDim.x)
+    ((double*)&o.obs)[k] = ((const double*)&sc->obs)[k];
+  if (threadIdx.x == 0) {
+    o.abort = sc->abort;
+    o.step = sc->step;
+    o.err = sc->err;
+  }
 }
 
 // Initial temperatures and Berendsen factors (main.F90:174-195).
