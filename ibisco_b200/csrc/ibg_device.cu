@@ -1536,7 +1536,7 @@ int ibg_create(const ibg_desc* d, int precision, ibg_ctx** out) {
     c->p_mom = dalloc<double>(3 * (size_t)c->g_mv, o);
     c->sc = dalloc<Scalars>(1, o);
     CK(cudaHostAlloc(&c->hsc, sizeof(Scalars), cudaHostAllocDefault));
-    c->ring_cap = 1;
+    c->ring_cap = 0;  // the first observed run allocates it
     c->ring = nullptr;
     refresh_args(c.get());
     CK(cudaDeviceSynchronize());
