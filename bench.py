@@ -731,9 +731,8 @@ def main():
                     help="centre-of-mass virtual sites: each at its centre of mass, or the reference's form "
                          "(VIRTUAL_DEF.f90:31 resets only the x sum)")
     ap.add_argument("--list-form", choices=["auto", "per-particle", "slice"], default="auto",
-                    help="Verlet lists of the FP32 single-system legs: the library's choice by list size, a list "
-                         "per particle, or one per slice of four slots with a pair mask per neighbour "
-                         "(ibg_set_list_form)")
+                    help="Verlet lists of the FP32 single-system legs: the library's choice, a list per particle, or one per "
+                         "slice of four slots with a pair mask per neighbour (ibg_set_list_form)")
     ap.add_argument("--precision", choices=["fp32", "fp64"], default="fp32")
     ap.add_argument("--no-cpu", action="store_true")
     ap.add_argument("--no-fp64", action="store_true")
