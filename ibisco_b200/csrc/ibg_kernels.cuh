@@ -436,8 +436,14 @@ struct ListArgs {
 };
 
 // List-rebuild kernels run when the step rebuilds its lists (or always, for
-// the rebuild of ibg_set_state) and the step is not skipped.
-//
+// the rebuild of ibg_set_state) and the step is not skipped.  The list builds
+// themselves raise skip when a slot outgrows the storage, while blocks of the
+// same launch may only be starting: there a block reads the flag together, so
+// that no warp leaves whose work the others wait for.
+__device__ __forceinline__ bool build_idle(const Scalars* sc, int always) {
+  return __syncthreads_or(sc->skip || !(always || sc->rebuild));
+}
+
 // Five launches: cells and counts, their scan, the cells' entries, their order
 // and new slots, the lists.  (They were eight; each costs ~4 us where the
 // system is small.)
@@ -706,7 +712,7 @@ __global__ void __launch_bounds__(256, 4) k_list_build_warp(__grid_constant__ co
   if (B) stage_args(&s_args, tab[bk.sys]);
   const ListArgs& L = B ? s_args : L0;
   Scalars* sc = L.sc;
-  if (sc->skip || !(always || sc->rebuild)) return;
+  if (build_idle(sc, always)) return;
   // candidates, 33 places per word: lanes that read different words at the
   // same time then hit different banks
   __shared__ PT s_pos[kWords * 33];
@@ -1000,7 +1006,7 @@ __global__ void __launch_bounds__(256) k_list_build_thread(__grid_constant__ con
   if (B) stage_args(&s_args, tab[bk.sys]);
   const ListArgs& L = B ? s_args : L0;
   Scalars* sc = L.sc;
-  if (sc->skip || !(always || sc->rebuild)) return;
+  if (build_idle(sc, always)) return;
   constexpr int P = 32 / T;
   __shared__ int s_ex[16][256];  // exclusions 5..20 of each thread's particle, as slots of this list
   __shared__ int s_late[kLateThread][256];  // each thread's entries of the outer group (rgroupsq), in order
@@ -1145,7 +1151,7 @@ __global__ void __launch_bounds__(256) k_list_build_slices(__grid_constant__ con
   if (B) stage_args(&s_args, tab[bk.sys]);
   const ListArgs& L = B ? s_args : L0;
   Scalars* sc = L.sc;
-  if (sc->skip || !(always || sc->rebuild)) return;
+  if (build_idle(sc, always)) return;
   constexpr int kWarps = 8;
   __shared__ int s_ex[kWarps][kUSlots][20];  // each particle's exclusions as slots of this list
   __shared__ int s_buf[kWarps][kUBuf];       // the slice's entries, in the order accepted
