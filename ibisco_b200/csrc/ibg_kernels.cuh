@@ -2286,10 +2286,12 @@ __device__ __forceinline__ void near_pair(const NBArgs<float>& A, const int4& nk
 
 // More pairs came at the cutoff than their buffer holds: record the need and
 // abort the step, which the host repeats with a larger buffer (as for the
-// Verlet-list storage).
+// Verlet-list storage).  Other threads of the launch may still be reading the
+// count: it stays as it is (the host clears it), so that whoever reads it takes
+// the same branch, and that branch leaves without a barrier, since a thread
+// that finds the skip flag raised has already left.
 __device__ __forceinline__ void near_overflow(Scalars* sc, int work, unsigned n) {
   sc->need_near[work] = (int)n;
-  sc->near_n[work] = 0u;
   sc->abort = 1;
   sc->skip = 1;
 }
@@ -2309,7 +2311,6 @@ __global__ void __launch_bounds__(256) k_nb_near(__grid_constant__ const NBArgs<
   if (A.near_in_collect || nb_idle(A)) return;
   const unsigned n = sc->near_n[A.work];
   if (n > (unsigned)A.near_cap) {
-    __syncthreads();  // every thread has read the count
     if (threadIdx.x == 0) near_overflow(sc, A.work, n);
     return;
   }
@@ -2383,7 +2384,6 @@ __global__ void __launch_bounds__(256, 4) k_nb_collect(__grid_constant__ const C
     if (near_n > 0) {
       const NBArgs<float>& A = *C.nb;
       if (near_n > (unsigned)A.near_cap) {
-        __syncthreads();  // every thread of the block has read the count
         if (bk.b == 0 && threadIdx.x == 0) near_overflow(sc, C.work, near_n);
         return;
       }
