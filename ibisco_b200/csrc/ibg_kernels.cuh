@@ -2548,9 +2548,11 @@ __device__ __forceinline__ void addf2(typename Prec<A>::acc_t* F, int i, const d
 // in a strained chain), while the terms are few; the forces are summed in the
 // path's accumulator (64-bit fixed point on the FP32 path).  Lengths and sines
 // that only scale a force are divided by through one reciprocal each (an angle
-// had 20 FP64 divisions, a torsion 27, of ~20 instructions; now 6 and 14); the
-// cosines of angles and dihedrals keep the reference's divisions, which their
-// arc cosine would amplify near straight and planar ones.  A particle's two
+// had 20 FP64 divisions, a torsion 27, of ~20 instructions; now 6 and 18).
+// Every cosine keeps the reference's divisions: the arc cosine amplifies its
+// rounding near straight angles and planar dihedrals, and a torsion's two bond
+// angles enter 1/sqrt(1 - cos^2), which does so by 1/sin^2 near straight ones
+// (two reciprocals in their place moved them by 3e-6 of the largest at 1e-5 rad).  A particle's two
 // shares of a term are added in one update.
 template <typename A, bool BA>
 __global__ void __launch_bounds__(256) k_bonded(__grid_constant__ const BondedArgs<A> B0, const BondedArgs<A>* const* tab,
@@ -2675,7 +2677,7 @@ __global__ void __launch_bounds__(256) k_bonded(__grid_constant__ const BondedAr
       if (rm > (R)0 || rm == (R)0) {
         for (int c = 0; c < 3; ++c) m[c] = m[c] / rm;
         iij = (R)1 / rij;
-        cosm = ((ij[0] * jk[0] + ij[1] * jk[1]) + ij[2] * jk[2]) * iij * ijk;
+        cosm = ((ij[0] * jk[0] + ij[1] * jk[1]) + ij[2] * jk[2]) / rij / rjk;
         isinm = (R)1 / r_sqrt((R)1 - cosm * cosm);
         cotanm = cosm * isinm;
       }
@@ -2690,7 +2692,7 @@ __global__ void __launch_bounds__(256) k_bonded(__grid_constant__ const BondedAr
       if (rn > (R)0 || rn == (R)0) {
         for (int c = 0; c < 3; ++c) nn[c] = nn[c] / rn;
         ikl = (R)1 / rkl;
-        cosn = ((jk[0] * kl[0] + jk[1] * kl[1]) + jk[2] * kl[2]) * ijk * ikl;
+        cosn = ((jk[0] * kl[0] + jk[1] * kl[1]) + jk[2] * kl[2]) / rjk / rkl;
         isinn = (R)1 / r_sqrt((R)1 - cosn * cosn);
         cotann = cosn * isinn;
       }
