@@ -2581,12 +2581,12 @@ __global__ void __launch_bounds__(256) k_bonded(__grid_constant__ const BondedAr
       const R rij = r_sqrt(rsq);
       const int t = e.z;
       const float4* T = B.tb + B.tb_off[t];
-      const R ibin = (R)1 / (R)B.tb_bin[t];
-      int k = fint((rij - (R)T[0].x) * ibin);
+      const R bin = (R)B.tb_bin[t];
+      int k = fint((rij - (R)T[0].x) / bin);  // the quotient: a length of whole bins decides the count below
       if (k > B.tb_ndat[t]) { ++overext; k = B.tb_ndat[t]; }
       else if (k < 0) k = 0;
       const float4 r0 = T[k], r1 = T[k + 1];
-      const R alpha = (rij - (R)r0.x) * ibin;
+      const R alpha = (rij - (R)r0.x) / bin;
       const R fij = lerp_mixed<R>((R)r0.y, (R)r1.y, alpha);
       const R vij = lerp_mixed<R>((R)r0.z, (R)r1.z, alpha);
       acc[e.w - 1] += (double)vij;

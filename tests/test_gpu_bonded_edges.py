@@ -64,3 +64,38 @@ def test_torsions_next_to_straight_angles(tmp_path):
     assert np.isfinite(fo).all() and np.abs(fo).max() > 1e5  # the sines are there
     assert rel_maxnorm(g.state64()["fxyz"], fo) < 1e-12
     assert og["V_TORSION1"] == pytest.approx(o.obs(1)["V_TORSION1"], rel=1e-12)
+
+
+@pytest.mark.parametrize("prec", [0, 1], ids=["fp32", "fp64"])
+def test_bonds_that_end_on_the_end_of_their_table(tmp_path, prec):
+    """A bond of exactly NDAT + 1 bins counts as overextended, one of NDAT bins
+    does not: the quotient length/bin is a whole number there, which the
+    length times 1/bin can miss (with two of the three tables it does)."""
+    bins = (0.0019, 0.001942, 0.002)
+    at = [np.array([c % 4, c // 4, 0]) * 1.8 - 2.7 for c in range(12)]
+    spec = chains(np.zeros((24, 3)), np.repeat(np.arange(12) % 3 + 1, 2), 3, 2, angle_tabs=[], torsion_tabs=[])
+    spec.bond_tabs = [((t + 1, t + 1), synth.harmonic_bond_table(f"bond{t}", 0.3, 1.0e3, 255 * b, b))
+                      for t, b in enumerate(bins)]
+    for c in range(12):  # x = 0 for the first of each pair, so that the difference is exact
+        spec.pos[2 * c] = spec.pos[2 * c + 1] = [0.0, at[c][0], at[c][1]]
+    d = synth.write_system(spec, str(tmp_path / "x"))
+    s = native.Setup(d)
+    b, nd = s.array("BINB").astype(np.float64), s.array("NDATB")
+    b, nd = b[-3:], nd[-3:]
+    assert list(nd) == [255] * 3
+    assert [256 * x * (1.0 / x) < 256 for x in b] == [True, True, False]
+    x, v, box = s.initial_state()
+    x = x.copy()
+    for c in range(12):
+        x[2 * c + 1, 0] = (256, 256, 255, 255)[c // 3] * b[c % 3]
+    g = native.System(s, prec)
+    g.set_state(x, v, box)
+    o = Oracle(d)
+    o.init(1)
+    o.set_state(x, v, box, 1)
+    og = g.forces(1)
+    o.forces(1, 1)
+    oo = o.obs(1)
+    assert oo["BOND_OVEREXT"] == 6
+    assert og["BOND_OVEREXT"] == 6
+    assert og["V_BOND1"] == pytest.approx(oo["V_BOND1"], rel=1e-12)
