@@ -1423,6 +1423,7 @@ struct NBArgs {
   // u = r/bin - (row within the table); one 16-byte read per pair
   const float4* tcoef;
   const double4* tcoef64;  // FP64 kernel: the same unscaled, in FP64
+  const double* rend;      // FP64 kernel, per type pair: the least r whose quotient r/bin is past NDAT
   const R* tx;
   int ntab, nrows;
   R rcutsq;
@@ -1597,10 +1598,15 @@ __global__ void __launch_bounds__(256, 2) k_nonbonded(__grid_constant__ const NB
       const int4 pt = pti[wj & 0xffff];
       const double r = r_sqrt(in ? G.r2 : 1.0);
       const double rb = r * __hiloint2double(pt.w, pt.z);
-      const int ni = fint(rb);
-      u = rb - (double)ni;
+      int ni = fint(rb);
       if (in && pt.x < 0) { err |= EB_MISSING_TABLE; in = false; }
-      if (in && (ni < 0 || ni > pt.y)) { err |= EB_TABLE_RANGE; in = false; }
+      if (in && (ni < 0 || ni >= pt.y)) {
+        // the last row: the quotient r/bin decides whether r is past the table
+        // (r times 1/bin can fall on the other side of a whole number of bins)
+        if (ni < 0 || r >= A.rend[ti * A.ntype + (wj & 0xffff)]) { err |= EB_TABLE_RANGE; in = false; }
+        ni = pt.y;
+      }
+      u = rb - (double)ni;
       return in ? pt.x + ni : 0;
     };
     auto pair = [&](const Geo& G, int t, int wj, const double4& co, double u) {
@@ -2552,7 +2558,8 @@ __device__ __forceinline__ void addf2(typename Prec<A>::acc_t* F, int i, const d
 // Every cosine keeps the reference's divisions: the arc cosine amplifies its
 // rounding near straight angles and planar dihedrals, and a torsion's two bond
 // angles enter 1/sqrt(1 - cos^2), which does so by 1/sin^2 near straight ones
-// (two reciprocals in their place moved them by 3e-6 of the largest at 1e-5 rad).  A particle's two
+// (with two reciprocals in their place forces were off by 3e-6 of the largest at
+// 1e-5 rad).  A particle's two
 // shares of a term are added in one update.
 template <typename A, bool BA>
 __global__ void __launch_bounds__(256) k_bonded(__grid_constant__ const BondedArgs<A> B0, const BondedArgs<A>* const* tab,
