@@ -1327,9 +1327,17 @@ long long ibg_device_bytes(const ibg_ctx* c) {
 long long ibg_estimate_bytes(const ibg_desc* d, int precision, const float* box) {
   if (!d || !box || d->nitems <= 0) return IBG_E_INVALID;
   const bool f32 = precision == IBG_PREC_FP32_FIXED;
-  const double pos = f32 ? 16.0 : 32.0, acc = 8.0, rs = f32 ? 4.0 : 8.0;
+  const double acc = 8.0;
+  // positions: a float4 and the box fractions, or a double4
+  const double pos = 32.0;
+  // table rows: {F, P}, X, the coefficients and, on one grid, their copy; or
+  // the FP64 coefficients
+  const double row = f32 ? 8.0 + 4.0 + 16.0 + 16.0 : 32.0;
   const double vol = (double)box[0] * box[1] * box[2];
-  double b = (double)d->nitems * (4 + 8 + 8 + 24 + 2 * 3 * acc + 4 + 80 + 4) + (double)d->natoms * 24;
+  // per particle: type word, mass and its inverse, state, both force sums,
+  // slot, exclusions, the buffer of the state's transfers; a site's members
+  double b = (double)d->nitems * (4 + 8 + 8 + 24 + 2 * 3 * acc + 4 + 80 + 4 + 48) + (double)d->natoms * 24 +
+             (double)d->nvirta * (3 * 4 + 15 * 12);
   long long terms = 0;
   for (int i = 0; i < d->nitems; ++i) {
     terms += d->nbonds ? d->nbonds[i] : 0;
@@ -1344,13 +1352,15 @@ long long ibg_estimate_bytes(const ibg_desc* d, int precision, const float* box)
     if (n <= 0) continue;
     const double rl = w == 0 ? d->rlist_atom : d->rlist_bead;
     const double half = (double)n / vol * (2.0 / 3.0) * 3.14159265358979 * rl * rl * rl;
-    const double rows = (half * 1.25 + 8.0) * 1.25 + 2.0;  // growth margin and slice padding
-    b += (double)n * (7 * 4 + 2 * pos + 3 * acc + rows * 4);
-    if (precision == IBG_PREC_FP32_FIXED) b += (double)n * 32 + 16.0 * std::max(4096, n / 32);  // box fractions, cutoff pairs
+    // the fullest particle's list in rows of 8 entries, with the growth margin
+    // of grow_lists; per particle: 7 integer arrays and its quarter of slice_w
+    const double rows = std::ceil((half * 1.25 + 8.0) / 8.0) * 1.25 + 2.0;
+    b += (double)n * (7 * 4 + 1 + pos + 3 * acc + rows * 8 * 4);
+    if (f32) b += 16.0 * std::max(4096, n / 32);  // pairs at the cutoff
     if (w == 1 && d->nmts > 0) b += (double)n * 9 * acc;
     const double cells = (box[0] * 1.25 / rl + 2) * (box[1] * 1.25 / rl + 2) * (box[2] * 1.25 / rl + 2);
-    b += cells * 12;
-    b += (double)d->nnbtype * d->ld_nb * 3 * rs;
+    b += cells * 8;
+    b += (double)d->nnbtype * d->ld_nb * row;
   }
   b += 2.0 * 1024 * 1024;  // scalars, partial sums, argument blocks, rounding of allocations
   return (long long)b;
