@@ -220,7 +220,7 @@ struct ibg_ctx {
   long long launches_per_variant[32] = {0};
   // graphs of several steps in a row, by their variants (run_steps)
   struct Chain {
-    cudaGraphExec_t exec = nullptr;  // captured when the sequence comes a second time
+    cudaGraphExec_t exec = nullptr;  // captured after the sequence came a second time
     long long launches = 0;
   };
   std::map<std::vector<unsigned char>, Chain> chains;
@@ -978,8 +978,15 @@ cudaGraphExec_t capture(ibg_ctx* c, long long* launches, F&& body) {
 // it the programmatic launch of the next step's first kernel overlaps the end
 // of the step before, where two graphs leave a gap (4,000-bead fluid 30.5 us a
 // step with a graph per step, 28.2 with ten; 40,000-bead melt 66.5 and 64.5).
-// The group is captured when its sequence of variants comes a second time, so
-// that a short run pays for no graph it does not use again.  Whole groups only:
+// A group whose sequence of variants came a second time is captured at the end
+// of that run, while the device works through it and the host would wait, and
+// only if it still does: capture and instantiation take 140 us (55 launches,
+// the fluid) to 900 us (103 and a second stream, the hybrid melt with MTS),
+// which the 17 to 22 us a replay saves on the melts would need some 20 replays
+// to earn.  The second stream takes the graph's upload (100 us in the next
+// run's first launch otherwise).  First run of 20 steps of a context, captured
+// where the sequence came again against here: 40,000-bead melt 1,810 and 1,435
+// us, hybrid NPT melt 2,020 and 1,570; later runs are the same.  Whole groups only:
 // their sequences repeat with the list, MTS and barostat periods (six with
 // lists every 10 steps and MTS 9), while runs of 24 steps cut into groups at
 // any step made 15 of them, captured again whenever the storage grew (hybrid
@@ -1750,6 +1757,7 @@ static int run_steps(ibg_ctx* c, int first, int nsteps, ibg_obs* per_step, bool 
       }
       CK(cudaEventRecord(c->run_ev[0], c->st));
       const int begin = done;
+      std::vector<std::pair<const std::vector<unsigned char>, ibg_ctx::Chain>*> again;  // groups to capture
       for (int k = begin; k < nsteps; ++k) {
         const int step = first + k;
         const bool flush = c->flush_bytes && c->flush_buf;
@@ -1760,16 +1768,13 @@ static int run_steps(ibg_ctx* c, int first, int nsteps, ibg_obs* per_step, bool 
             auto it = c->chains.find(key);
             if (it == c->chains.end()) {
               if (c->chains.size() < kMaxChains) c->chains.emplace(key, ibg_ctx::Chain{});
-            } else {
-              ibg_ctx::Chain& ch = it->second;
-              if (!ch.exec)
-                ch.exec = capture(c, &ch.launches, [&] {
-                  for (int q = 0; q < kChain; ++q) enqueue(c, key[q], q > 0);
-                });
-              CK(cudaGraphLaunch(ch.exec, c->st));
-              c->launches += ch.launches;
+            } else if (it->second.exec) {
+              CK(cudaGraphLaunch(it->second.exec, c->st));
+              c->launches += it->second.launches;
               k += kChain - 1;
               continue;
+            } else {
+              again.push_back(&*it);
             }
           }
         }
@@ -1793,6 +1798,20 @@ static int run_steps(ibg_ctx* c, int first, int nsteps, ibg_obs* per_step, bool 
       // one read-back per run: step, abort and error flags, observables
       CK(cudaMemcpyAsync(c->hsc, c->sc, sizeof(Scalars), cudaMemcpyDeviceToHost, c->st));
       collect_marks(c);
+      // (kChain) groups are captured here, where the host would only wait
+      for (auto* g : again) {
+        if (g->second.exec) continue;
+        const cudaError_t e = cudaEventQuery(c->run_ev[1]);
+        if (e != cudaErrorNotReady) {
+          CK(e);
+          break;
+        }
+        (void)cudaGetLastError();
+        g->second.exec = capture(c, &g->second.launches, [&] {
+          for (int q = 0; q < kChain; ++q) enqueue(c, g->first[q], q > 0);
+        });
+        CK(cudaGraphUpload(g->second.exec, c->st2));
+      }
       CK(cudaStreamSynchronize(c->st));
       float ms = 0.f;
       CK(cudaEventElapsedTime(&ms, c->run_ev[0], c->run_ev[1]));
