@@ -978,20 +978,23 @@ cudaGraphExec_t capture(ibg_ctx* c, long long* launches, F&& body) {
 // it the programmatic launch of the next step's first kernel overlaps the end
 // of the step before, where two graphs leave a gap (4,000-bead fluid 30.5 us a
 // step with a graph per step, 28.2 with ten; 40,000-bead melt 66.5 and 64.5).
-// A group whose sequence of variants came a second time is captured at the end
-// of that run, while the device works through it and the host would wait, and
-// only if it still does: capture and instantiation take 140 us (55 launches,
+// A group whose sequence of variants comes a second time is captured, but only
+// while the device has work: capture and instantiation take 140 us (55 launches,
 // the fluid) to 900 us (103 and a second stream, the hybrid melt with MTS),
 // which the 17 to 22 us a replay saves on the melts would need some 20 replays
-// to earn.  The second stream takes the graph's upload (100 us in the next
-// run's first launch otherwise).  First run of 20 steps of a context, captured
-// where the sequence came again against here: 40,000-bead melt 1,810 and 1,435
-// us, hybrid NPT melt 2,020 and 1,570; later runs are the same.  Whole groups only:
+// to earn.  So a run that has queued kAhead steps or more (0.5 ms of the
+// fluid, 1.2 of the 40,000-bead melt) captures at once, a shorter one at its
+// end, where the host would only wait; there the second stream takes the
+// graph's upload (100 us in the next run's first launch otherwise).  First run
+// of 20 steps of a context, captured where the sequence came again against at
+// the end: 40,000-bead melt 1,810 and 1,435 us, hybrid NPT melt 2,020 and
+// 1,570; later runs are the same.  Whole groups only:
 // their sequences repeat with the list, MTS and barostat periods (six with
 // lists every 10 steps and MTS 9), while runs of 24 steps cut into groups at
 // any step made 15 of them, captured again whenever the storage grew (hybrid
 // melt 3.67 ms a run against 3.17).  kMaxChains bounds how many are kept.
 constexpr int kChain = 10;
+constexpr int kAhead = 20;
 constexpr size_t kMaxChains = 32;
 
 // The system runs steps step_before+1 .. last; observables of step k go to
@@ -1757,7 +1760,13 @@ static int run_steps(ibg_ctx* c, int first, int nsteps, ibg_obs* per_step, bool 
       }
       CK(cudaEventRecord(c->run_ev[0], c->st));
       const int begin = done;
-      std::vector<std::pair<const std::vector<unsigned char>, ibg_ctx::Chain>*> again;  // groups to capture
+      using Group = std::pair<const std::vector<unsigned char>, ibg_ctx::Chain>;
+      std::vector<Group*> again;  // groups to capture at the end
+      auto take = [&](Group& g) {
+        g.second.exec = capture(c, &g.second.launches, [&] {
+          for (int q = 0; q < kChain; ++q) enqueue(c, g.first[q], q > 0);
+        });
+      };
       for (int k = begin; k < nsteps; ++k) {
         const int step = first + k;
         const bool flush = c->flush_bytes && c->flush_buf;
@@ -1768,12 +1777,14 @@ static int run_steps(ibg_ctx* c, int first, int nsteps, ibg_obs* per_step, bool 
             auto it = c->chains.find(key);
             if (it == c->chains.end()) {
               if (c->chains.size() < kMaxChains) c->chains.emplace(key, ibg_ctx::Chain{});
-            } else if (it->second.exec) {
-              CK(cudaGraphLaunch(it->second.exec, c->st));
-              c->launches += it->second.launches;
-              k += kChain - 1;
-              continue;
             } else {
+              if (!it->second.exec && k - begin >= kAhead) take(*it);
+              if (it->second.exec) {
+                CK(cudaGraphLaunch(it->second.exec, c->st));
+                c->launches += it->second.launches;
+                k += kChain - 1;
+                continue;
+              }
               again.push_back(&*it);
             }
           }
@@ -1807,9 +1818,7 @@ static int run_steps(ibg_ctx* c, int first, int nsteps, ibg_obs* per_step, bool 
           break;
         }
         (void)cudaGetLastError();
-        g->second.exec = capture(c, &g->second.launches, [&] {
-          for (int q = 0; q < kChain; ++q) enqueue(c, g->first[q], q > 0);
-        });
+        take(*g);
         CK(cudaGraphUpload(g->second.exec, c->st2));
       }
       CK(cudaStreamSynchronize(c->st));
