@@ -289,7 +289,8 @@ size_t possize(const ibg_ctx* c) { return c->prec == IBG_PREC_FP32_FIXED ? sizeo
 // The list form of a list of n particles.  Automatic choice: per-particle
 // lists.  Measured with slice lists beside them, per step with lists rebuilt
 // every 10 steps: the 2,000,000-bead melt 1.473 against 1.721 ms, a
-// 160,000-bead melt 164 against 170 us, the 40,000-bead melt 69.6 against 69.3.
+// 160,000-bead melt 164 against 170 us, the 40,000-bead melt 69.6 against 69.3
+// (no difference beyond the runs').
 int list_form_of(const ibg_ctx* c, int n) {
   if (c->prec != IBG_PREC_FP32_FIXED || n >= (1 << 28)) return IBG_LIST_PER_PARTICLE;
   return c->list_form == IBG_LIST_PER_SLICE ? IBG_LIST_PER_SLICE : IBG_LIST_PER_PARTICLE;
@@ -488,8 +489,8 @@ void build_list(ibg_ctx* c, const ibg_desc* d, int which) {
     L.ptab = dupload(pt, o);
     L.rend = dupload(rend, o);
   }
-  // launch default: tables read through L1 (staged, the FP64 kernel's launch on
-  // the 40,000-bead melt takes 82 us instead of 59)
+  // launch default: tables read through L1 (staged, a launch takes as long on
+  // the melts, on both paths, and 61 to 69 us instead of 52 on the hybrid melt)
   L.use_smem = false;
 }
 
@@ -585,7 +586,7 @@ void make_args(ibg_ctx* c) {
     n.pos4 = L.pos4; n.posq = L.posq; n.counts = L.counts; n.slice_w = L.slice_w; n.entries = L.entries;
     n.w_cap = L.w_cap; n.work = w;
     n.fsort = (acc_t*)L.fsort;
-    n.tfp = (const R*)L.tfp; n.tx = (const R*)L.tx; n.ptab = L.ptab; n.chunk = sizeof(R) == 4 ? c->nb_chunk : 24;  // the FP64 path has no choice of it
+    n.tfp = (const R*)L.tfp; n.tx = (const R*)L.tx; n.ptab = L.ptab; n.chunk = sizeof(R) == 4 ? c->nb_chunk : 24;  // fixed on the FP64 path
     n.tcoef = L.tcoef; n.tcoef64 = L.tcoef64; n.rend = L.rend; n.pbase = L.pbase; n.tuni = L.tuni; n.uinv = L.uinv; n.r2_none = L.r2_none; n.urows = L.urows;
     n.rows = c->nb_rows;
     n.window = c->nb_window;
@@ -731,8 +732,10 @@ struct NBKey {
 };
 // Blocks of 512 threads for one system over lists with tables on one grid:
 // 32 warps per SM as with 256, but twice as many of them share one range of
-// slices, and with it the positions in L1 (160,000-bead melt 101 us a launch
-// against 105, hybrid melt 82 against 85).  A batch hands blocks to systems,
+// slices, and with it the positions in L1 (launches between events, 512 against
+// 256: 2,000,000-bead melt 1,019 and 1,028 us, hybrid melt 52.7 and 54.4,
+// 40,000-bead melt 32.6 and 32.7, 160,000-bead melt 94.6 and 92.5).  A batch
+// hands blocks to systems,
 // and its kernel holds the argument block in shared memory: 384 threads at 80
 // registers, without the 140 bytes of spills it has at 64 (24 mixed jobs 6.39
 // ms per 20 steps against 6.51).
@@ -1396,8 +1399,8 @@ int ibg_create(const ibg_desc* d, int precision, ibg_ctx** out) {
     // launch defaults (ibg_set_tuning / ibg_autotune change them).  FP32 path:
     // a block's own range of units, the last 24/256 shared out; with every unit
     // taken from the global counter (0) the nonbonded launch of the
-    // 2,000,000-bead melt takes 1,234 us instead of 871, of a 160,000-bead one
-    // 99 instead of 90
+    // 2,000,000-bead melt takes 1,834 us instead of 1,019, of a 160,000-bead one
+    // 125 instead of 95, of the 40,000-bead melt 42 instead of 33
     c->nb_chunk = precision == IBG_PREC_FP32_FIXED ? 24 : 0;
     c->natoms = d->natoms; c->nvirta = d->nvirta; c->nitems = d->nitems; c->ntype = d->ntype;
     c->numatoms = d->numatoms; c->numbeads = d->numbeads; c->ncoarse = d->ncoarse;

@@ -678,18 +678,17 @@ static const int kStencilHost[13][3] = IBG_HALF_STENCIL;  // the same, for host 
 // other shift the distance is above RLIST either way.  A cell none of whose
 // runs wrapped has no shifts to subtract.
 //
-// Bound by instruction issue (160,000-bead melt: ~310 warp instructions a
-// particle for the distances, ~370 for writing the entries, the rest for
-// staging, exclusions and counts).  A warp per particle that tests 32
+// Bound by its block barriers and by instruction issue (ncu, 40,000-bead melt:
+// 40 % of the stalls at barriers, issue 57 %; 160,000-bead melt: ~310 warp
+// instructions a particle for the distances, ~370 for writing the entries, the
+// rest for staging, exclusions and counts).  A warp per particle that tests 32
 // candidates at a time took ~1,400 (two ballots, prefix counts, exclusion
 // compares and the shift for every 32 tests): launch 276 us, now ~220; the
-// hybrid melt's two lists 405 us a rebuild with the cell sort, now 252.
+// hybrid melt's two lists 405 us a rebuild with the cell sort, now 246.
 // Entries written by a lane per candidate, word by word, took 450 a particle;
 // by a lane per word, 1,150 (the words next to the particle are full).
 //
-// Candidates a block stages: 1,536 in FP32, 768 in FP64.  A staged slot carries
-// its run (0..13) in bits 27..30, so lists hold fewer than 2^27 particles.
-constexpr int kSlotMask = (1 << 27) - 1;
+// Candidates a block stages: 1,536 in FP32, 768 in FP64.
 // Entries of the outer group a thread of the thread-per-particle build holds
 // back to append after the others.
 constexpr int kLateThread = 24;
@@ -968,8 +967,9 @@ __global__ void __launch_bounds__(256, 4) k_list_build_warp(__grid_constant__ co
 }
 
 // NEW_NEIGHBOUR_WITHLIST.f90:34-123 for large lists: a thread builds one
-// particle's list (k_list_build_warp, above, gives a warp to each particle and
-// suits lists too short to fill the GPU with one thread per particle).
+// particle's list (k_list_build_warp, above, gives a block to up to 32 particles
+// of a cell and suits lists too short to fill the GPU with one thread per
+// particle).
 // A warp takes 32 consecutive slots at a time (dynamically), so its lanes
 // mostly share a cell and walk the same candidates in step: a candidate's
 // position is one load that the lanes share, and each lane appends what it
@@ -1506,7 +1506,9 @@ struct NbUnits {
 // coefficients (A + B u, C + D u); two rows are evaluated in step and units are
 // handed out as in k_nonbonded_f32.  16 warps per SM at 128 registers: at 24
 // warps (80 registers, 108 bytes of spills) the launch took 189 us on the
-// 160,000-bead melt, with 16 174 (before: 216), without the block ranges.
+// 160,000-bead melt, with 16 174 (before: 216), all without the block ranges.
+// Between events, caches as the step leaves them: 182 us there, 52 on the
+// 40,000-bead melt, with the tables staged or not.
 template <bool SMEM, int T, bool B>
 __global__ void __launch_bounds__(256, 2) k_nonbonded(__grid_constant__ const NBArgs<double> A0,
                                                       const NBArgs<double>* const* tab, const BlockMap bm) {
@@ -1686,8 +1688,8 @@ __global__ void __launch_bounds__(256, 2) k_nonbonded(__grid_constant__ const NB
 // fabsf(fij) r below 0.99 kFixMax, tested on the force scaled by 2^32
 constexpr float kFixLimScaled = 0.99f * kFixMax * kFixScale;
 // The FP32 nonbonded kernels' energy and virial sums, at the start of their
-// dynamic shared memory: 7 per lane of their 256-thread blocks for a list of
-// one label, 9 for a list of several.  A lane adds to its own words, with no
+// dynamic shared memory: 7 per lane of their blocks for a list of one label, 9
+// for a list of several.  A lane adds to its own words, with no
 // shuffle and no half-idle warp (per pair of lanes, they took 16 shuffles and
 // nine half-warp updates for every eight list rows).
 __host__ __device__ constexpr int nb_acc_bytes(bool mixed, int nt) { return (mixed ? 9 : 7) * nt * (int)sizeof(long long); }
@@ -1766,12 +1768,16 @@ __device__ __forceinline__ void nb_block_sums(const NBArgs<float>& A, long long*
 // and two table rows are in flight per lane; a pair that does not count reads
 // a row of zeros instead of branching; lanes keep their own energy and virial
 // sums; the next unit's header is loaded ahead.  58.2 M -> 47 M warp
-// instructions, launch 105 -> 87 us; with blocks of 512 threads and a unit per
-// slice the 2,000,000-bead melt's launch went from 1,131 to 868 us.  Measured
-// and dropped: tables staged in shared memory (99.2 against 99.5 us: random
-// 16-byte rows conflict on banks as they do on L1 tags), positions fetched a
-// row pair ahead (spills at 64 registers, 24 warps at 80: 100 us), units dealt
-// to warps statically (94 against 88 us: uneven slices).
+// instructions.  A launch, between events, caches as the step leaves them:
+// 40,000-bead melt 33 us, 160,000 beads 94, the hybrid melt's atoms and sites 52,
+// 2,000,000 beads with k_nb_near 1,010 (ncu, cold caches, without it: 1,131
+// before, 963 now).  Measured and dropped: positions fetched a row pair ahead
+// (spills at 64 registers, 24 warps at 80: 101 and 100 against 99 us on 160,000
+// beads, each beside the kernel of its day), units dealt to warps statically (94
+// against 88: uneven slices).  Tables staged in shared memory gain nothing
+// (random 16-byte rows conflict on banks as they do on L1 tags: 40,000-bead
+// melt 32.8 against 32.6, hybrid melt 61 to 69 against 52); they stay a choice
+// of the caller's.
 template <bool SMEM, bool MIXED, bool UNI, bool B, int NT>
 __global__ void __launch_bounds__(NT, 1024 / NT) k_nonbonded_f32(__grid_constant__ const NBArgs<float> A0,
                                                           const NBArgs<float>* const* tab, const BlockMap bm) {

@@ -76,10 +76,13 @@ __device__ __forceinline__ long long fixq(float v, unsigned* err) {
 // Bound by the latency of its dependent loads (LIST, then the neighbour's
 // position and type, then its table rows): with one thread per A a list of
 // ~50 neighbours was one chain of ~150 of them, and 3,000 particles kept 12
-// blocks busy.  Whole call, a thread per A against 32 and 8 lanes: 3,001
-// particles 154 us, 70, 79; 30,000 146, 96, 104; 60,000 170, 134, 128; 100,000
-// 198, 154, 157.  So a list of fewer than kWideLists particles takes a warp
-// each, a longer one eight lanes (their neighbours share sectors of LIST).
+// blocks busy (whole call of 3,001 particles 154 us, of 100,000 198).  Whole
+// call, 32 against 8 lanes (medians of four runs each): 1,000 particles 71 and
+// 75 us, 3,001 74 and 76, 20,000 87 and 95, 30,000 96 and 97, the same within 1 %
+// from 37,000 (103) over 100,000 (157) to 215,000 (232), 262,144 287 and 274.  So
+// a list of fewer than kWideLists particles takes a warp each, a longer one
+// eight lanes (their neighbours share sectors of LIST); the line may lie
+// anywhere between 37,000 and 215,000.
 constexpr int kWideLists = 45000;
 template <int T>
 __global__ void __launch_bounds__(256) k_static_pairs(StaticArgs a) {

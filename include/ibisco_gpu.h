@@ -230,7 +230,8 @@ int ibg_set_list_rows(ibg_ctx* c, int rows);
    neighbour's position and adds its force once per slice.  Lists rebuilt
    every 10 steps, a step with per-particle lists takes 1.47 ms on the
    2,000,000-bead melt (slice lists 1.72 ms) and 164 us on a 160,000-bead one
-   (170 us).  IBG_LIST_AUTO (the default): per-particle lists.  Changing
+   (170 us); on 40,000 beads both take 69 us.  IBG_LIST_AUTO (the default):
+   per-particle lists.  Changing
    the form discards the stored lists: ibg_set_state must be called again
    before the next step.  ibg_get_list_form returns the form in use (of the
    atom list, or of the bead list when there is no atom list):
@@ -241,13 +242,16 @@ int ibg_set_list_rows(ibg_ctx* c, int rows);
 int ibg_set_list_form(ibg_ctx* c, int form);
 int ibg_get_list_form(const ibg_ctx* c);
 /* Launch tuning of the nonbonded kernel: nb_tables_smem stages the tables in
-   shared memory per block (1) or reads them through L1 (0, the default);
+   shared memory per block (1) or reads them through L1 (0, the default).
+   Tables that take more than 200 KB with the kernel's sums (32 bytes a row on
+   the FP64 path, 16 on the FP32 path) stay in L1, and ibg_get_tuning returns 0;
    nb_blocks_per_sm limits the resident blocks per SM (0: all that fit);
    nb_chunk (FP32 path; default 24): each block works through its own
    contiguous range of work units (neighbouring slices), so its warps gather
    from one region of space, and the last nb_chunk/256 of the units are taken
    dynamically by whichever warps finish first (0: every warp takes units
-   alone, dynamically); nb_rows: list rows per work unit, 8 or 16 (0: 16);
+   alone, dynamically; the FP64 path always has ranges and 24, and reads back
+   0); nb_rows: list rows per work unit, 8 or 16 (0: 16);
    nb_window (FP32 path, nb_chunk > 0): 0 gives each block one contiguous range
    of units, W > 0 deals runs of W consecutive units to the blocks in turn, so
    that all blocks work through one region of space at a time.  Forces and
