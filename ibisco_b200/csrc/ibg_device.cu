@@ -795,7 +795,10 @@ int nb_occupancy(const ibg_ctx* c, const DevList& L, size_t sm) {
   (void)c;
   const NBKey key = nb_key(L, B);
   NBKernel<R, B> k = nb_kernel<R, B>(key);
-  if (sm > 48 * 1024) CK(cudaFuncSetAttribute((const void*)k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
+  // the same limit for every context: the attribute is the kernel's, and a
+  // smaller one would refuse the launches of a context with larger tables
+  if (sm > 48 * 1024)
+    CK(cudaFuncSetAttribute((const void*)k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemLimit));
   int per = 0;
   CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, (const void*)k, key.nt, sm));
   per = std::max(1, per);
