@@ -139,7 +139,6 @@ struct DevList {
   bool uni = false;
   void *tfp = nullptr, *tx = nullptr;  // FP32 path
   double4* tcoef64 = nullptr;          // FP64 path (NBArgs::tcoef64)
-  double* rend = nullptr;              // FP64 path (NBArgs::rend)
   float4* tcoef = nullptr;  // FP32 path: per row {F - dF e, P - dP e, dF, dP} (NBArgs::tcoef)
   int ntab = 0, nrows = 0;
   bool use_smem = false;  // tables staged in shared memory (tuning)
@@ -469,25 +468,32 @@ void build_list(ibg_ctx* c, const ibg_desc* d, int which) {
         co[k].x = fk - df * e; co[k].y = pk - dp * e; co[k].z = df; co[k].w = dp;
       }
     L.tcoef64 = dupload(co, o);
-    std::vector<double> end(L.ntab, 0.0), rend(pt.size(), 0.0);
+    // The kernel takes r times 1/bin for the quotient r/bin.  At the table's end
+    // the quotient decides between a row and an error, and the product can fall
+    // on the other side of the whole number: 1/bin is moved by a rounding or two
+    // where that is so, up until the least distance past the table is past it in
+    // the product too, else down until the one below is not (that one double may
+    // stay past it, in a tenth of all tables).  (A test of r itself in the kernel
+    // took 178 us a launch instead of 173 on the 160,000-bead melt.)
+    std::vector<double> inv(L.ntab);
     for (int t = 0; t < L.ntab; ++t) {
+      inv[t] = 1.0 / bin[t];
       const double past = tnd[t] + 1.0;
-      if (!(bin[t] > 0.0)) continue;
-      double r = past * bin[t];
-      while (r > 0.0 && r / bin[t] >= past) r = std::nextafter(r, 0.0);
-      while (!(r / bin[t] >= past)) r = std::nextafter(r, HUGE_VAL);
-      end[t] = r;
+      if (!(bin[t] > 0.0 && std::isfinite(bin[t]))) continue;
+      double end = past * bin[t];  // the least r with r/bin past the table
+      while (end > 0.0 && end / bin[t] >= past) end = std::nextafter(end, 0.0);
+      while (!(end / bin[t] >= past)) end = std::nextafter(end, HUGE_VAL);
+      while (end * inv[t] < past) inv[t] = std::nextafter(inv[t], HUGE_VAL);
+      while (std::nextafter(end, 0.0) * inv[t] >= past && end * std::nextafter(inv[t], 0.0) >= past)
+        inv[t] = std::nextafter(inv[t], 0.0);
     }
     for (size_t k = 0; k < pt.size(); ++k) {
       const int t = ltab[k];
-      if (t >= 0) rend[k] = end[t];
-      const double inv = t >= 0 ? 1.0 / bin[t] : 0.0;
-      int ib[2];
-      std::memcpy(ib, &inv, sizeof(inv));
+      int ib[2] = {0, 0};
+      if (t >= 0) std::memcpy(ib, &inv[t], sizeof(double));
       pt[k] = t >= 0 ? make_int4(toff[t], tnd[t], ib[0], ib[1]) : make_int4(-1, 0, 0, 0);
     }
     L.ptab = dupload(pt, o);
-    L.rend = dupload(rend, o);
   }
   // launch default: tables read through L1 (staged, a launch takes as long on
   // the melts, on both paths, and 61 to 69 us instead of 52 on the hybrid melt)
@@ -587,7 +593,7 @@ void make_args(ibg_ctx* c) {
     n.w_cap = L.w_cap; n.work = w;
     n.fsort = (acc_t*)L.fsort;
     n.tfp = (const R*)L.tfp; n.tx = (const R*)L.tx; n.ptab = L.ptab; n.chunk = sizeof(R) == 4 ? c->nb_chunk : 24;  // fixed on the FP64 path
-    n.tcoef = L.tcoef; n.tcoef64 = L.tcoef64; n.rend = L.rend; n.pbase = L.pbase; n.tuni = L.tuni; n.uinv = L.uinv; n.r2_none = L.r2_none; n.urows = L.urows;
+    n.tcoef = L.tcoef; n.tcoef64 = L.tcoef64; n.pbase = L.pbase; n.tuni = L.tuni; n.uinv = L.uinv; n.r2_none = L.r2_none; n.urows = L.urows;
     n.rows = c->nb_rows;
     n.window = c->nb_window;
     n.ntab = L.ntab; n.nrows = L.nrows; n.rcutsq = (R)L.rcutsq;

@@ -1423,7 +1423,6 @@ struct NBArgs {
   // u = r/bin - (row within the table); one 16-byte read per pair
   const float4* tcoef;
   const double4* tcoef64;  // FP64 kernel: the same unscaled, in FP64
-  const double* rend;      // FP64 kernel, per type pair: the least r whose quotient r/bin is past NDAT
   const R* tx;
   int ntab, nrows;
   R rcutsq;
@@ -1507,7 +1506,7 @@ struct NbUnits {
 // handed out as in k_nonbonded_f32.  16 warps per SM at 128 registers: at 24
 // warps (80 registers, 108 bytes of spills) the launch took 189 us on the
 // 160,000-bead melt, with 16 174 (before: 216), all without the block ranges.
-// Between events, caches as the step leaves them: 182 us there, 52 on the
+// Between events, caches as the step leaves them: 174 us there, 50.5 on the
 // 40,000-bead melt, with the tables staged or not.
 template <bool SMEM, int T, bool B>
 __global__ void __launch_bounds__(256, 2) k_nonbonded(__grid_constant__ const NBArgs<double> A0,
@@ -1600,15 +1599,10 @@ __global__ void __launch_bounds__(256, 2) k_nonbonded(__grid_constant__ const NB
       const int4 pt = pti[wj & 0xffff];
       const double r = r_sqrt(in ? G.r2 : 1.0);
       const double rb = r * __hiloint2double(pt.w, pt.z);
-      int ni = fint(rb);
-      if (in && pt.x < 0) { err |= EB_MISSING_TABLE; in = false; }
-      if (in && (ni < 0 || ni >= pt.y)) {
-        // the last row: the quotient r/bin decides whether r is past the table
-        // (r times 1/bin can fall on the other side of a whole number of bins)
-        if (ni < 0 || r >= A.rend[ti * A.ntype + (wj & 0xffff)]) { err |= EB_TABLE_RANGE; in = false; }
-        ni = pt.y;
-      }
+      const int ni = fint(rb);
       u = rb - (double)ni;
+      if (in && pt.x < 0) { err |= EB_MISSING_TABLE; in = false; }
+      if (in && (ni < 0 || ni > pt.y)) { err |= EB_TABLE_RANGE; in = false; }
       return in ? pt.x + ni : 0;
     };
     auto pair = [&](const Geo& G, int t, int wj, const double4& co, double u) {
