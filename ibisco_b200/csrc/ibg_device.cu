@@ -248,6 +248,7 @@ int fail(ibg_ctx* c, int code, const std::string& m) {
 
 // The captured step graphs: they hold the argument blocks by value.
 void drop_graphs(ibg_ctx* c) {
+  if (!c->chains.empty()) cudaStreamSynchronize(c->st2);  // an upload on its way (run_steps)
   for (auto& kv : c->graphs) cudaGraphExecDestroy(kv.second);
   for (auto& kv : c->chains)
     if (kv.second.exec) cudaGraphExecDestroy(kv.second.exec);
