@@ -288,7 +288,7 @@ size_t possize(const ibg_ctx* c) { return c->prec == IBG_PREC_FP32_FIXED ? sizeo
 // ----------------------------------------------------------- list setup
 // The list form of a list of n particles.  Automatic choice: per-particle
 // lists.  Measured with slice lists beside them, per step with lists rebuilt
-// every 10 steps: the 2,000,000-bead melt 1.473 against 1.721 ms, a
+// every 10 steps: the 2,000,000-bead melt 1.521 against 1.687 ms, a
 // 160,000-bead melt 164 against 170 us, the 40,000-bead melt 69.6 against 69.3
 // (no difference beyond the runs').
 int list_form_of(const ibg_ctx* c, int n) {

@@ -228,11 +228,10 @@ int ibg_set_list_rows(ibg_ctx* c, int rows);
    pairs, so ibg_get_neighbour_list returns the same LIST and NNEBS and every
    force sum is bit for bit the same; the slice form gathers each stored
    neighbour's position and adds its force once per slice.  Lists rebuilt
-   every 10 steps, a step with per-particle lists takes 1.47 ms on the
-   2,000,000-bead melt (slice lists 1.72 ms) and 164 us on a 160,000-bead one
+   every 10 steps, a step with per-particle lists takes 1.52 ms on the
+   2,000,000-bead melt (slice lists 1.69 ms) and 164 us on a 160,000-bead one
    (170 us); on 40,000 beads both take 69 us.  IBG_LIST_AUTO (the default):
-   per-particle lists.  Changing
-   the form discards the stored lists: ibg_set_state must be called again
+   per-particle lists.  Changing the form discards the stored lists: ibg_set_state must be called again
    before the next step.  ibg_get_list_form returns the form in use (of the
    atom list, or of the bead list when there is no atom list):
    IBG_LIST_PER_PARTICLE or IBG_LIST_PER_SLICE. */
