@@ -1765,10 +1765,10 @@ __device__ __forceinline__ void nb_block_sums(const NBArgs<float>& A, long long*
 // instructions.  A launch, between events, caches as the step leaves them:
 // 40,000-bead melt 33 us, 160,000 beads 94, the hybrid melt's atoms and sites 52,
 // 2,000,000 beads with k_nb_near 1,010 (ncu, cold caches, without it: 1,131
-// before, 963 now).  Measured and dropped: positions fetched a row pair ahead
-// (spills at 64 registers, 24 warps at 80: 101 and 100 against 99 us on 160,000
-// beads, each beside the kernel of its day), units dealt to warps statically (94
-// against 88: uneven slices).  Tables staged in shared memory gain nothing
+// before, 963 now).  Measured and dropped on 160,000 beads, each beside the kernel
+// of its day: positions fetched a row pair ahead (107 us with spills at 64
+// registers, 100 at 80 and 24 warps, against 101), units dealt to warps
+// statically (94 against 88: uneven slices).  Tables staged in shared memory gain nothing
 // (random 16-byte rows conflict on banks as they do on L1 tags: 40,000-bead
 // melt 32.8 against 32.6, hybrid melt 61 to 69 against 52); they stay a choice
 // of the caller's.
